@@ -1,0 +1,181 @@
+// Device memory of the engine: growing buffers, and the pool of the instance
+// that the C API drives.
+#pragma once
+
+#include <cuda_runtime_api.h>
+#include <stddef.h>
+#include <stdint.h>
+
+#include <memory>
+#include <utility>
+#include <vector>
+
+namespace tb {
+
+// Device bytes of the engine whose calls this thread is running (the
+// serving form's admission accounting); null: not counted.
+extern thread_local long long* g_dbuf_account;
+// When set, buffers are allocated and freed stream-ordered on this stream
+// (cudaMallocAsync / cudaFreeAsync), so engines that run side by side on their
+// own streams never wait for each other's frees; null: cudaMalloc / cudaFree.
+extern thread_local cudaStream_t g_dbuf_stream;
+// With g_dbuf_stream: the pool the stream-ordered allocations come from
+// (null: the device's current pool).
+extern thread_local cudaMemPool_t g_dbuf_pool;
+
+// Device memory of one engine: a memory pool of its own, for the instance that
+// the C API drives.  A new mesh needs about 200 buffers, which cost 90 us each
+// with cudaMalloc and 80 us with cudaFree; the pool maps device memory in
+// larger pieces.  It keeps up to kKeep bytes that no buffer uses and goes back
+// to the device with the engine's last buffer.
+//
+// A buffer may be used on any of the streams that the engine's work runs on
+// (users).  It goes back to the pool, on the pool's own stream, after
+// everything that is on them when it is let go: nothing is handed out again
+// while a kernel may still read it, and no other work on the device is waited
+// for.  Where that order cannot be had (a user stream is being captured), the
+// buffer is held until it can.
+struct DevPool {
+  static constexpr uint64_t kKeep = 512ull << 20;
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t st = nullptr;
+  cudaEvent_t ev = nullptr;
+  int device = -1;
+  std::vector<cudaStream_t> users;  // (empty: nothing of the engine is running any more)
+  std::vector<void*> held;          // let go, and not back in the pool yet
+  DevPool() {
+    if (cudaGetDevice(&device) != cudaSuccess) return;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = kKeep;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) pool = nullptr;
+    if (pool && (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+                 cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
+                 cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)) {
+      if (st) cudaStreamDestroy(st);
+      cudaMemPoolDestroy(pool);
+      pool = nullptr;
+    }
+    if (!pool) cudaGetLastError();
+  }
+  ~DevPool() {
+    if (!pool) return;
+    give_back();
+    cudaStreamSynchronize(st);
+    cudaMemPoolDestroy(pool);
+    cudaEventDestroy(ev);
+    cudaStreamDestroy(st);
+  }
+  DevPool(const DevPool&) = delete;
+  DevPool& operator=(const DevPool&) = delete;
+  // false: the caller asks the device directly (which then has what the pool
+  // did not use)
+  bool alloc(void** p, size_t bytes) {
+    int d = -1;
+    if (!pool || cudaGetDevice(&d) != cudaSuccess || d != device) return false;
+    give_back();
+    if (cudaMallocFromPoolAsync(p, bytes, pool, st) == cudaSuccess) {
+      if (cudaStreamSynchronize(st) == cudaSuccess) return true;
+      cudaFreeAsync(*p, st);
+    }
+    cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    return false;
+  }
+  void free(void* p) {
+    held.push_back(p);
+    give_back();
+  }
+
+ private:
+  void give_back() {
+    if (held.empty() || !after_users()) return;
+    for (void* p : held) cudaFreeAsync(p, st);
+    held.clear();
+  }
+  // the pool's stream goes on after everything on the users' streams
+  bool after_users() {
+    for (cudaStream_t s : users) {
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;  // (an event of a capture would draw st into it)
+      if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+          cudaEventRecord(ev, s) != cudaSuccess || cudaStreamWaitEvent(st, ev, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+    }
+    return true;
+  }
+};
+// The pool of the instance whose calls this thread makes; empty, or with
+// g_dbuf_stream: none.
+extern thread_local std::weak_ptr<DevPool> g_dbuf_dev;
+
+template <class T>
+struct DBuf {
+  T* p = nullptr;
+  size_t n = 0;
+  long long* acct = nullptr;  // where this allocation is counted
+  cudaStream_t st = nullptr;  // stream-ordered allocation: its stream
+  bool async = false;
+  std::shared_ptr<DevPool> dev;  // or: the pool it comes from
+  DBuf() = default;
+  DBuf(const DBuf&) = delete;
+  DBuf& operator=(const DBuf&) = delete;
+  DBuf(DBuf&& o) noexcept { swap(o); }
+  DBuf& operator=(DBuf&& o) noexcept {
+    swap(o);
+    return *this;
+  }
+  ~DBuf() { release(); }
+  void swap(DBuf& o) {
+    std::swap(p, o.p);
+    std::swap(n, o.n);
+    std::swap(acct, o.acct);
+    std::swap(st, o.st);
+    std::swap(async, o.async);
+    std::swap(dev, o.dev);
+  }
+  cudaError_t ensure(size_t count) {
+    if (count <= n && p) return cudaSuccess;
+    // a buffer that has to grow again gets a quarter more, so slowly growing
+    // sizes (moving meshes) do not reallocate every call
+    const size_t grow = (p && count) ? count / 4 : 0;
+    release();
+    size_t c = count ? count + grow : 1;
+    const size_t bytes = c * sizeof(T);
+    async = g_dbuf_stream != nullptr;
+    st = g_dbuf_stream;
+    if (!async) dev = g_dbuf_dev.lock();
+    if (dev && !dev->alloc((void**)&p, bytes)) dev.reset();
+    cudaError_t e = dev           ? cudaSuccess
+                    : !async      ? cudaMalloc((void**)&p, bytes)
+                    : g_dbuf_pool ? cudaMallocFromPoolAsync((void**)&p, bytes, g_dbuf_pool, st)
+                                  : cudaMallocAsync((void**)&p, bytes, st);
+    if (e == cudaSuccess) {
+      n = c;
+      acct = g_dbuf_account;
+      if (acct) *acct += (long long)bytes;
+    } else {
+      p = nullptr;
+    }
+    return e;
+  }
+  void release() {
+    if (p) {
+      if (dev) dev->free(p);
+      else if (async) cudaFreeAsync(p, st);
+      else cudaFree(p);
+      if (acct) *acct -= (long long)(n * sizeof(T));
+    }
+    p = nullptr;
+    n = 0;
+    acct = nullptr;
+    async = false;
+    dev.reset();
+    st = nullptr;
+  }
+};
+
+}  // namespace tb

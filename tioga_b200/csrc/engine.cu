@@ -71,14 +71,16 @@ Engine::~Engine() {
   for (auto& e : up_slot_ev_) cudaEventDestroy(e);
   h_tab_.release();
   h_rb_.release();
-  // (the device buffers, then their stream, go with the members)
-  if (dev_pool_) dev_pool_->idle = dev_pool_->wait();
+  // (the device buffers, then their stream, go with the members; nothing uses
+  // them any more)
+  if (dev_pool_) dev_pool_->users.clear();
 }
 
 // Work on the caller's stream (nullptr: back to the library's own stream).
 void Engine::set_stream(cudaStream_t s) {
   cudaStreamSynchronize(stream_);
   stream_ = s ? s : own_stream_;
+  if (dev_pool_) dev_pool_->users = {stream_, side_, up_};
 }
 
 int Engine::find_tag(int tag) const { return find_block(cur_sys_, tag); }

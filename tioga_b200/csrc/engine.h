@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "devmem.h"
 
 namespace tb {
 
@@ -47,150 +48,6 @@ constexpr int kMaxBlocks = 100; // MAXBLOCKS, src/globals.h:29
 constexpr int kMaxSysBlocks = 16;      // blocks of one overset system (donor lists per node)
 constexpr int kMaxEngineBlocks = 8192;
 constexpr size_t kHoleMapCap = 197ull * 197ull * 197ull;  // bytes of one hole map at most // blocks of all systems of one engine (16-bit block ids)
-
-// Device bytes of the engine whose calls this thread is running (the
-// serving form's admission accounting); null: not counted.
-extern thread_local long long* g_dbuf_account;
-// When set, buffers are allocated and freed stream-ordered on this stream
-// (cudaMallocAsync / cudaFreeAsync), so engines that run side by side on their
-// own streams never wait for each other's frees; null: cudaMalloc / cudaFree.
-extern thread_local cudaStream_t g_dbuf_stream;
-// With g_dbuf_stream: the pool the stream-ordered allocations come from
-// (null: the device's current pool).
-extern thread_local cudaMemPool_t g_dbuf_pool;
-
-// Device memory of one engine: a memory pool of its own, for the instance that
-// the C API drives.  A new mesh needs about 200 buffers, which cost 90 us each
-// with cudaMalloc and 80 us with cudaFree; the pool maps device memory in
-// larger pieces (a new mesh of 450 k nodes from registration to its first data
-// update and the end of the instance: 50 ms, 30 ms with it).  It keeps up to kKeep bytes that no buffer uses and goes back
-// to the device with the engine's last buffer.  As with cudaFree, a buffer is
-// let go only when the device is idle, so it may be used on any stream.
-struct DevPool : std::enable_shared_from_this<DevPool> {
-  static constexpr uint64_t kKeep = 512ull << 20;
-  cudaMemPool_t pool = nullptr;
-  cudaStream_t st = nullptr;
-  int device = -1;
-  bool idle = false;  // the engine is going: nothing of it is running any more
-  DevPool() {
-    if (cudaGetDevice(&device) != cudaSuccess) return;
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    uint64_t keep = kKeep;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) pool = nullptr;
-    if (pool && (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
-                 cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess)) {
-      cudaMemPoolDestroy(pool);
-      pool = nullptr;
-    }
-    if (!pool) cudaGetLastError();
-  }
-  ~DevPool() {
-    if (!pool) return;
-    cudaStreamSynchronize(st);
-    cudaMemPoolDestroy(pool);
-    cudaStreamDestroy(st);
-  }
-  DevPool(const DevPool&) = delete;
-  DevPool& operator=(const DevPool&) = delete;
-  // false: the caller asks the device directly (which then has what the pool
-  // did not use)
-  bool alloc(void** p, size_t bytes) {
-    int d = -1;
-    if (!pool || cudaGetDevice(&d) != cudaSuccess || d != device) return false;
-    if (cudaMallocFromPoolAsync(p, bytes, pool, st) == cudaSuccess) {
-      if (cudaStreamSynchronize(st) == cudaSuccess) return true;
-      cudaFreeAsync(*p, st);
-    }
-    cudaGetLastError();
-    cudaMemPoolTrimTo(pool, 0);
-    return false;
-  }
-  void free(void* p) {
-    if (!idle) wait();
-    cudaFreeAsync(p, st);
-  }
-  // until the pool's device is idle, whichever device is the thread's
-  bool wait() {
-    int d = -1;
-    if (cudaGetDevice(&d) != cudaSuccess) return false;
-    if (d != device) cudaSetDevice(device);
-    const bool ok = cudaDeviceSynchronize() == cudaSuccess;
-    if (d != device) cudaSetDevice(d);
-    return ok;
-  }
-};
-// The pool of the instance whose calls this thread makes; empty, or with
-// g_dbuf_stream: none.
-extern thread_local std::weak_ptr<DevPool> g_dbuf_dev;
-
-template <class T>
-struct DBuf {
-  T* p = nullptr;
-  size_t n = 0;
-  long long* acct = nullptr;  // where this allocation is counted
-  cudaStream_t st = nullptr;  // stream-ordered allocation: its stream
-  bool async = false;
-  std::shared_ptr<DevPool> dev;  // or: the pool it comes from
-  DBuf() = default;
-  DBuf(const DBuf&) = delete;
-  DBuf& operator=(const DBuf&) = delete;
-  DBuf(DBuf&& o) noexcept { swap(o); }
-  DBuf& operator=(DBuf&& o) noexcept {
-    swap(o);
-    return *this;
-  }
-  ~DBuf() { release(); }
-  void swap(DBuf& o) {
-    std::swap(p, o.p);
-    std::swap(n, o.n);
-    std::swap(acct, o.acct);
-    std::swap(st, o.st);
-    std::swap(async, o.async);
-    std::swap(dev, o.dev);
-  }
-  cudaError_t ensure(size_t count) {
-    if (count <= n && p) return cudaSuccess;
-    // a buffer that has to grow again gets a quarter more, so slowly growing
-    // sizes (moving meshes) do not reallocate every call
-    const size_t grow = (p && count) ? count / 4 : 0;
-    release();
-    size_t c = count ? count + grow : 1;
-    const size_t bytes = c * sizeof(T);
-    async = g_dbuf_stream != nullptr;
-    st = g_dbuf_stream;
-    if (!async) dev = g_dbuf_dev.lock();
-    if (dev && !dev->alloc((void**)&p, bytes)) dev.reset();
-    cudaError_t e = dev           ? cudaSuccess
-                    : !async      ? cudaMalloc(&p, bytes)
-                    : g_dbuf_pool ? cudaMallocFromPoolAsync((void**)&p, bytes, g_dbuf_pool, st)
-                                  : cudaMallocAsync((void**)&p, bytes, st);
-    if (e == cudaSuccess) {
-      n = c;
-      acct = g_dbuf_account;
-      if (acct) *acct += (long long)bytes;
-    } else {
-      p = nullptr;
-    }
-    return e;
-  }
-  void release() {
-    if (p) {
-      if (dev) dev->free(p);
-      else if (async) cudaFreeAsync(p, st);
-      else cudaFree(p);
-      if (acct) *acct -= (long long)(n * sizeof(T));
-    }
-    p = nullptr;
-    n = 0;
-    acct = nullptr;
-    async = false;
-    dev.reset();
-    st = nullptr;
-  }
-};
 
 // Page-locked host memory that grows: copies to and from it do not hold the
 // host (a 4-byte read-back into pageable memory costs 14 us, into this 5).
@@ -395,7 +252,10 @@ struct Timing {
 class Engine {
  public:
   std::weak_ptr<DevPool> dev_pool() {
-    if (!dev_pool_) dev_pool_ = std::make_shared<DevPool>();
+    if (!dev_pool_) {
+      dev_pool_ = std::make_shared<DevPool>();
+      dev_pool_->users = {stream_, side_, up_};
+    }
     return dev_pool_;
   }
   // high-order path
