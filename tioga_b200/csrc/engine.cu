@@ -2521,6 +2521,11 @@ int Engine::dataupdate(int nvar, int interptype) {
     fprintf(stderr, "#tioga_b200: register every block's solution on the same side (host or device)\n");
     return -1;
   }
+  if (nvar < 0) {
+    fprintf(stderr, "#tioga_b200: data update of %d fields\n", nvar);
+    return -1;
+  }
+  if (nvar == 0) return 0;
   TB_CUDA(qvals_.ensure((size_t)nrec_ * nvar));
   const long long nval = nrec_ * nvar;
   if (device) {
