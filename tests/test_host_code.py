@@ -20,3 +20,8 @@ def test_buffers_go_back_after_the_work_that_reads_them(tmp_path):
     captured."""
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     _run(tmp_path, "devmem_check.cc", "g++", "-I", os.path.join(cuda, "include"))
+
+
+def test_donor_slots_refuse_indices_outside_their_arrays(tmp_path):
+    """Both kernels that fill the donor slots take their places from here."""
+    _run(tmp_path, "donor_slots_check.cu", os.environ.get("NVCC", "nvcc"))

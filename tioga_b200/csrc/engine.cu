@@ -1428,8 +1428,9 @@ int Engine::run_search() {
   // still to come changes outcomes, so the slots wait for it)
   slots_filled_ = !any_uhex_ && !dedup_ran_;
   k_search_finish<<<grid_for(nq_, kT), kT, 0, stream_>>>(qkey_.p, qacc_.p, nq_, inv_sorted_.p, qcell_.p, qtie_.p,
-                                                         qnode_.p, qdon_.p, K_, d_bi_.p,
-                                                         slots_filled_ ? slot_.p : nullptr, counters_.p);
+                                                         qnode_.p, qdon_.p,
+                                                         slots_filled_ ? donor_slots() : DonorSlots{}, counters_.p,
+                                                         err_.p);
   TB_LAUNCHED("k_search_finish");
   if (any_uhex_) {  // donors that are uniform boxes: the index lookup (search.C:271-341)
     k_uhex_search<<<grid_for(nq_, kT), kT, 0, stream_>>>(x_.p, qnode_.p, qdon_.p, nq_, d_bi_.p, uhex_map_.p,
@@ -1779,8 +1780,7 @@ int Engine::run_donors() {
   // candidate slots: one per (receptor node, donor block)
   if (nq_ > 0) {
     if (!slots_filled_) {
-      k_fill_slots<<<grid_for(nq_, kT), kT, 0, stream_>>>(qnode_.p, qdon_.p, qcell_.p, nq_, K_, ntot_, ctot_,
-                                                          d_bi_.p, (int)hb_.size(), slot_.p, err_.p);
+      k_fill_slots<<<grid_for(nq_, kT), kT, 0, stream_>>>(qnode_.p, qdon_.p, qcell_.p, nq_, donor_slots(), err_.p);
       TB_LAUNCHED("k_fill_slots");
     }
     k_classify_queried<<<grid_for(nq_, kT), kT, 0, stream_>>>(x_.p, node_blk_.p, d_bi_.p, slot_.p, K_, qnode_.p,

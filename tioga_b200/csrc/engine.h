@@ -104,6 +104,23 @@ struct BlockInfo {
   float bb_lo[3], bb_hi[3];  // block box for the Morton keys
 };
 
+// The donor slots: one per node and block of its system, the query whose donor
+// is in that block (-1: none).
+struct DonorSlots {
+  int* slot;
+  int K;  // slots per node
+  long long ntot, ctot;
+  const BlockInfo* bi;
+  int nb;
+  // the place of a query with node g and donor cell c of block d; -1 where an
+  // index is outside its array
+  __host__ __device__ long long at(int g, int d, int c) const {
+    if (g < 0 || g >= ntot || d < 0 || d >= nb || c < 0 || c >= ctot) return -1;
+    const int a = d - bi[d].sblk0;  // the donor's index within its system
+    return a < 0 || a >= K ? -1 : (long long)g * K + a;
+  }
+};
+
 struct PairInfo {  // one (receptor block, donor block) pair, src/exchangeBoxes.C:133-160
   int rec, don;
   double rd[6];    // reduced box accumulator in the donor's OBB frame (ordered bits)
@@ -411,6 +428,7 @@ class Engine {
   int download_iblank();
   int fetch_interps();
   int find_tag(int tag) const;
+  DonorSlots donor_slots() const { return {slot_.p, K_, ntot_, ctot_, d_bi_.p, (int)hb_.size()}; }
 
   std::vector<HostBlock> hb_;
   std::vector<BlockInfo> bi_;

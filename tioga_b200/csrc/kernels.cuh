@@ -175,8 +175,7 @@ __global__ void k_refine(const double* x, const int* conn8, const unsigned char*
                          const unsigned* nrefine, unsigned long long* qkey, unsigned* qacc);
 __global__ void k_search_finish(const unsigned long long* qkey, const unsigned* qacc, long long nq,
                                 const int* inv_sorted, int* qcell, unsigned char* qtie, const int* qnode,
-                                const int* qdon, int K, const BlockInfo* bi, int* slot,
-                                unsigned long long* counters);
+                                const int* qdon, DonorSlots slots, unsigned long long* counters, unsigned* err);
 
 // ---- uniform-hex fast path (kernels_uhex.cu) ----
 __global__ void k_uhex_check(const double* x, const int* conn8, const BlockInfo* bi, int b, double d0, double d1,
@@ -190,8 +189,8 @@ __global__ void k_uhex_search(const double* x, const int* qnode, const int* qdon
                               unsigned char* qtie);
 
 // ---- donors (kernels_donor.cu) ----
-__global__ void k_fill_slots(const int* qnode, const int* qdon, const int* qcell, long long nq, int K,
-                             long long ntot, long long ctot, const BlockInfo* bi, int nb, int* slot, unsigned* err);
+__global__ void k_fill_slots(const int* qnode, const int* qdon, const int* qcell, long long nq, DonorSlots slots,
+                             unsigned* err);
 __global__ void k_donor_rest(long long ntot, long long ctot, int K, unsigned char* m0, int* m1, int* cmark, int* reset_t,
                              int* slot, int* iblank_cell, int* dcnt);
 __global__ void k_write_iblanks(const int* iblank, const blk_t* node_blk, long long ntot, int* const* dst);

@@ -2359,13 +2359,13 @@ __global__ void __launch_bounds__(128) k_refine(const double* __restrict__ x, co
   }
 }
 
-// Search, stage 4: per query outcome and tie flags; with slot, also the donor
-// slots (k_fill_slots, when no later kernel changes an outcome).
+// Search, stage 4: per query outcome and tie flags; with slots, also the donor
+// slots (as k_fill_slots, when no later kernel changes an outcome).
 __global__ void k_search_finish(const unsigned long long* __restrict__ qkey, const unsigned* __restrict__ qacc,
                                 long long nq, const int* __restrict__ inv_sorted, int* __restrict__ qcell,
                                 unsigned char* __restrict__ qtie, const int* __restrict__ qnode,
-                                const int* __restrict__ qdon, int K, const BlockInfo* __restrict__ bi,
-                                int* __restrict__ slot, unsigned long long* __restrict__ counters) {
+                                const int* __restrict__ qdon, DonorSlots slots,
+                                unsigned long long* __restrict__ counters, unsigned* __restrict__ err) {
   unsigned long long my_tie = 0, my_found = 0;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq;
        q += (long long)gridDim.x * blockDim.x) {
@@ -2378,7 +2378,11 @@ __global__ void k_search_finish(const unsigned long long* __restrict__ qkey, con
     qtie[q] = tie;
     my_tie += (tie != 0);
     my_found += (donor >= 0);
-    if (slot && donor >= 0) slot[(long long)qnode[q] * K + qdon[q] - bi[qdon[q]].sblk0] = (int)q;
+    if (slots.slot && donor >= 0) {
+      const long long at = slots.at(qnode[q], qdon[q], donor);
+      if (at < 0) atomicOr(err, kErrBadIndex);
+      else slots.slot[at] = (int)q;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     my_tie += __shfl_xor_sync(0xffffffffu, my_tie, o);

@@ -40,20 +40,15 @@ __device__ __forceinline__ int donor_list(long long g, const int* __restrict__ s
 }
 
 __global__ void k_fill_slots(const int* __restrict__ qnode, const int* __restrict__ qdon,
-                             const int* __restrict__ qcell, long long nq, int K, long long ntot,
-                             long long ctot, const BlockInfo* __restrict__ bi, int nb, int* __restrict__ slot,
+                             const int* __restrict__ qcell, long long nq, DonorSlots slots,
                              unsigned* __restrict__ err) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq;
        q += (long long)gridDim.x * blockDim.x) {
     const int c = qcell[q];
     if (c < 0) continue;
-    const int g = qnode[q], d = qdon[q];
-    const int a = (d >= 0 && d < nb) ? d - bi[d].sblk0 : -1;  // the donor's index within its system
-    if (c >= ctot || g < 0 || g >= ntot || a < 0 || a >= K) {
-      atomicOr(err, kErrBadIndex);
-      continue;
-    }
-    slot[(long long)g * K + a] = (int)q;
+    const long long at = slots.at(qnode[q], qdon[q], c);
+    if (at < 0) atomicOr(err, kErrBadIndex);
+    else slots.slot[at] = (int)q;
   }
 }
 
