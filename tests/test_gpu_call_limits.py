@@ -53,3 +53,23 @@ def test_update_of_no_fields(side, oracle_lib):
     for b, a in zip(system.blocks, q):
         assert np.array_equal(a.cpu().numpy().view(np.int64), ref["q"][b.tag].view(np.int64))
     t.delete()
+
+
+def test_phase_times_are_the_connectivity_calls():
+    """Elements described after a connectivity call have every cell boxed
+    again; the times read afterwards are still those of the call."""
+    system, ho = cases.small_config4()
+    t = _connected(system)
+    tb.set_int(t.lib, "tioga_b200_set_coords_resident_", 1)
+    t.performconnectivity()
+    assert tb.stats(t.lib)["boxed_cells"] > 0
+    for b, h in zip(system.blocks, ho):
+        x = np.ascontiguousarray(h.xdof)
+        t._keep.append(x)
+        t.lib.tioga_b200_set_highorder_lagrange_(C.byref(C.c_int(b.tag)), C.byref(C.c_int(h.p)),
+                                                 x.ctypes.data_as(C.c_void_p))
+    t.lib.tioga_performconnectivity_highorder_()
+    assert t.lib.tioga_b200_last_error() == 0
+    ms = tb.timing(t.lib)
+    t.delete()
+    assert 0 < ms["holemap"] < ms["total"] and 0 < ms["cell_boxes"] < ms["cell_pass"] < ms["boxes_refit"], ms

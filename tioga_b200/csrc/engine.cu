@@ -1353,6 +1353,7 @@ int Engine::launch_refit(cudaStream_t st) {
 // (the pairs come out as they are: the boxes are what this is for)
 int Engine::all_cell_boxes() {
   if (!groups_culled_) return 0;
+  fetch_timing();  // the call's own times: the events are recorded anew below
   boxes_ready_ = tiles_ready_ = false;
   TB_TRY(run_pairs_and_refit());
   TB_CUDA(cudaStreamWaitEvent(stream_, rf_ev_, 0));
