@@ -73,3 +73,63 @@ def test_phase_times_are_the_connectivity_calls():
     ms = tb.timing(t.lib)
     t.delete()
     assert 0 < ms["holemap"] < ms["total"] and 0 < ms["cell_boxes"] < ms["cell_pass"] < ms["boxes_refit"], ms
+
+
+DELTA = 10.0 / 2 ** 19  # the coincidence gate's distance in a block 10 wide
+
+
+def _graded(inner, gap, twin=None):
+    """A box 10 wide whose inner nodes per axis lie `gap` apart around the
+    origin, under a shell; with `twin` another node there, moved from a node
+    of the box by that much."""
+    a = (np.arange(inner) - 0.5 * (inner - 1)) * gap
+    far = np.geomspace(a[-1] + gap, 5.0, 6)
+    ax = np.concatenate([-far[::-1], a, far])
+    n = len(ax)
+    x, cells = cases.hex_box(n, -5.0, 5.0)
+    ijk = np.rint((x + 5.0) * (n - 1) / 10.0).astype(int)
+    x = ax[ijk]
+    if twin is not None:
+        mid = np.flatnonzero((ijk == n // 2).all(1))[0]
+        x = np.concatenate([x, x[mid:mid + 1] + np.array([[0.0, twin, 0.0]])])
+    none = np.zeros(0, np.int32)
+    xs, cs, wall, outer, _ = cases.sphere_shell(9, 9, 17, 0.5, 2.0, 1.1, np.array([1.0, 0.2, 0.1]), 0.0,
+                                                np.random.default_rng(0))
+    return cases.System([cases.Block(1, np.ascontiguousarray(x), cells, none, none),
+                         cases.Block(2, xs, cs, wall, outer)])
+
+
+def _preprocess_ms(t):
+    import time
+    best = 1e9
+    for _ in range(4):
+        t0 = time.perf_counter()
+        t.preprocess_grids()
+        best = min(best, 1e3 * (time.perf_counter() - t0))
+    return best
+
+
+@pytest.mark.parametrize("inner,gap", [(17, 1.03), (30, 2.1), (44, 7.0)])
+def test_coincidence_gate_of_graded_blocks(inner, gap, oracle_lib):
+    """Thousands of nodes in a cell of the coincidence gate, none closer than
+    its distance: no merge runs and a preprocess costs what it costs on a mesh
+    of as many nodes that is not graded.  With one node closer than that (and
+    within TOL) the merge runs and merges it."""
+    plain = cases.config0(3, nbg=inner + 12, nr=9, nt=9, nphi=17, perturb=0.0)
+    t = _connected(plain)
+    plain_launches, plain_ms = tb.stats(t.lib)["launches"], _preprocess_ms(t)
+    t.delete()
+    for twin in (None, 1e-12, -0.3 * DELTA):
+        system = _graded(inner, gap * DELTA, twin)
+        ref = run_system(oracle_lib, system)
+        t = _connected(system)
+        st = tb.stats(t.lib)
+        assert (st["nmerged"] > 0) == (twin == 1e-12)
+        assert (st["launches"] > plain_launches + 10) == (twin is not None), (st["launches"], plain_launches)
+        for b in system.blocks:
+            assert np.array_equal(ref["iblank"][b.tag], t.iblank(b.tag))
+            for a, c in zip(ref["donors"][b.tag], t.getdonorinfo(b.tag)):
+                assert np.array_equal(a, c)
+        ms = _preprocess_ms(t)
+        t.delete()
+        assert ms < 6 * plain_ms, (ms, plain_ms)

@@ -987,9 +987,10 @@ int Engine::preprocess() {
   TB_CUDA(cudaStreamSynchronize(stream_));
   memcpy(bi_.data(), h_rb_.p, bi_bytes);
   if (gate) {
-    unsigned close_nodes;
-    memcpy(&close_nodes, h_rb_.p + bi_bytes, sizeof(unsigned));
-    dedup_active_ = close_nodes != 0;
+    unsigned found;
+    memcpy(&found, h_rb_.p + bi_bytes, sizeof(unsigned));
+    dedup_active_ = (found & 1u) != 0;
+    if (found == 2u) TB_TRY(dedup_gate_crowded(&dedup_active_));
   }
   if (fresh || tree_nodes_ == 0) {
     TB_TRY(build_tree_topology());  // also puts the cell arrays in storage order
@@ -1503,7 +1504,8 @@ int Engine::traverse_and_gather(const double* xq, const int* qn, const int* qd, 
 // without such nodes cannot produce query points within TOL of each other,
 // and the per-call merge is skipped.  Nodes farther apart than the gate
 // distance at preprocess that later move within TOL of each other are not
-// merged until the next preprocess.  The flag is read with the boxes.
+// merged until the next preprocess.  The flag is read with the boxes: bit 0
+// close nodes, bit 1 a crowded block (dedup_gate_crowded then decides).
 int Engine::dedup_gate() {
   unsigned mask = 1023;  // entries: 1.2 per node; the table at most half full
   while ((long long)mask + 1 < 2 * ntot_ + ntot_ / 2) mask = 2 * mask + 1;
@@ -1515,6 +1517,23 @@ int Engine::dedup_gate() {
   k_coin_hash<<<grid_for(ntot_, kT), kT, 0, stream_>>>(x_.p, node_blk_.p, d_bi_.p, ntot_, node_bin_.p, cg_table_.p,
                                                        mask, cg_flag_.p);
   TB_LAUNCHED("k_coin_hash");
+  return 0;
+}
+
+int Engine::dedup_gate_crowded(bool* close) {
+  unsigned mask = 1023;  // an entry per node: at most 0.4 full
+  while ((long long)mask + 1 < 2 * ntot_ + ntot_ / 2) mask = 2 * mask + 1;
+  TB_CUDA(cudaMemsetAsync(cg_table_.p, 0xff, ((size_t)mask + 1) * sizeof(int), stream_));
+  TB_CUDA(cudaMemsetAsync(cg_flag_.p, 0, sizeof(unsigned), stream_));
+  k_coin_file<<<grid_for(ntot_, kT), kT, 0, stream_>>>(x_.p, node_blk_.p, d_bi_.p, ntot_, cg_table_.p, mask,
+                                                       cg_flag_.p);
+  TB_LAUNCHED("k_coin_file");
+  k_coin_compare<<<grid_for(ntot_, kT), kT, 0, stream_>>>(x_.p, node_blk_.p, d_bi_.p, ntot_, cg_table_.p, mask,
+                                                          cg_flag_.p);
+  TB_LAUNCHED("k_coin_compare");
+  TB_CUDA(cudaMemcpyAsync(h_rb_.p, cg_flag_.p, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_));
+  TB_CUDA(cudaStreamSynchronize(stream_));
+  *close = *reinterpret_cast<const unsigned*>(h_rb_.p) != 0;
   return 0;
 }
 

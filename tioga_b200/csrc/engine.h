@@ -417,6 +417,7 @@ class Engine {
   int run_donors();
   int donor_rest_init();
   int dedup_gate();
+  int dedup_gate_crowded(bool* close);
   int run_dedup();
   int dedup_merge(const DedupQueries& Q, const std::vector<int>& qoff);
   int traverse_and_gather(const double* xq, const int* qn, const int* qd, long long nq, unsigned& count,

@@ -226,6 +226,10 @@ __global__ void k_interp(const double* x, const unsigned long long* rkey, const 
                          unsigned* err);
 __global__ void k_coin_hash(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot, short* node_bin,
                             int* table, unsigned mask, unsigned* flag);
+__global__ void k_coin_file(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot, int* table,
+                            unsigned mask, unsigned* flag);
+__global__ void k_coin_compare(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot,
+                               const int* table, unsigned mask, unsigned* flag);
 __global__ void k_dedup_keys(const int* qnode, const int* qdon, long long nq, const int* pair_qoff, int npairs,
                              const int* pair_rank, const short* node_bin, int node_bits, unsigned long long* key,
                              int* val);

@@ -58,10 +58,44 @@ __device__ __forceinline__ short node_bin_of(const double p[3], const Obb& o) {
 // nodes; sorting the (cell, node) list instead took 13 launches and 24 bytes
 // of traffic per node and radix pass (a host step of 340 k nodes 2722 us with
 // it, 2482 us now; of 6 k nodes 1056 and 902 us).
+//
+// On a strongly graded block (nodes a few delta apart in a far field 10^5 of
+// them wide) a filing cell holds thousands of nodes.  A walk longer than any on
+// an ordinary mesh (at a table half full of 20 M entries the longest is about
+// 25) therefore ends the pass as crowded, and the host has the gate decided on
+// cells 2 delta wide instead: nodes that are not closer than delta lie at most
+// some dozens in such a cell, whatever the mesh.  Each is filed once, under its
+// own cell (k_coin_file), and then looks through the cells that its delta-box
+// touches (k_coin_compare).  30^3 nodes two delta apart: a preprocess 0.30 ms; it
+// took 29 ms with walks of up to 4096, and 0.55 ms with the sorted list.
 // ---------------------------------------------------------------------------
 constexpr int kCoinBits = 17;      // delta is a quarter of a cell of 2^17 per axis (at least 10 TOL)
 constexpr int kCoinCoarse = 8;     // width of a filing cell in those cells
-constexpr int kCoinProbes = 4096;  // a longer walk counts as a hit (the merge then runs, to the same result)
+constexpr int kCoinWalk = 128;     // a longer walk counts as crowded
+constexpr double kCoinFine = 2.01; // width of a crowded gate's cells in delta
+constexpr int kCoinProbes = 4096;  // there a longer walk counts as close nodes (the merge then runs, to the same result)
+constexpr unsigned kCoinClose = 1u, kCoinCrowded = 2u;  // the gate's flag
+
+// delta of a block, and a cell's place in the table
+__device__ __forceinline__ double coin_delta(const BlockInfo& B) {
+  double ext = 0;
+  for (int k = 0; k < 3; k++) ext = fmax(ext, (double)B.bb_hi[k] - (double)B.bb_lo[k]);
+  return 0.25 * fmax(ext / (double)(1 << kCoinBits), 40.0 * kTol);
+}
+__device__ __forceinline__ void coin_place(int b, int i, int j, int k, unsigned mask, unsigned& at, unsigned& step) {
+  unsigned long long h = ((unsigned long long)b << 51) ^ ((unsigned long long)i << 34) ^ ((unsigned long long)j << 17) ^
+                         (unsigned long long)k;
+  h *= 0x9E3779B97F4A7C15ull;  // Fibonacci hashing: the high bits
+  at = (unsigned)(h >> 32) & mask;
+  step = (unsigned)(h >> 13) | 1u;  // (odd: the walk meets every entry)
+}
+__device__ __forceinline__ bool coin_close(const double* __restrict__ x, const blk_t* __restrict__ node_blk,
+                                           const double p[3], int g, int b, int other, double delta) {
+  const double* o = x + 3ll * other;  // (both loads under way at once)
+  const int ob = node_blk[other];
+  const double d = fabs(p[0] - o[0]) + fabs(p[1] - o[1]) + fabs(p[2] - o[2]);
+  return other != g && ob == b && d < delta;
+}
 
 __global__ void k_coin_hash(const double* __restrict__ x, const blk_t* __restrict__ node_blk,
                             const BlockInfo* __restrict__ bi, long long ntot, short* __restrict__ node_bin,
@@ -73,9 +107,7 @@ __global__ void k_coin_hash(const double* __restrict__ x, const blk_t* __restric
     const BlockInfo& B = bi[b];
     const double p[3] = {x[3 * g], x[3 * g + 1], x[3 * g + 2]};
     node_bin[g] = node_bin_of(p, B.obb);
-    double ext = 0;
-    for (int k = 0; k < 3; k++) ext = fmax(ext, (double)B.bb_hi[k] - (double)B.bb_lo[k]);
-    const double s = fmax(ext / (double)(1 << kCoinBits), 40.0 * kTol), delta = 0.25 * s, inv = 1.0 / (kCoinCoarse * s);
+    const double delta = coin_delta(B), inv = 1.0 / (4 * kCoinCoarse * delta);
     constexpr double reach = 0.2501 / kCoinCoarse;  // delta in filing cells, with room for the rounding of t
     int c0[3], n[3];
     for (int k = 0; k < 3; k++) {
@@ -92,27 +124,77 @@ __global__ void k_coin_hash(const double* __restrict__ x, const blk_t* __restric
       at[m] = step[m] = 0;
       old[m] = -1;
       if (i < n[0] && j < n[1] && k < n[2]) {
-        unsigned long long h = ((unsigned long long)b << 51) ^ ((unsigned long long)(c0[0] + i) << 34) ^
-                               ((unsigned long long)(c0[1] + j) << 17) ^ (unsigned long long)(c0[2] + k);
-        h *= 0x9E3779B97F4A7C15ull;  // Fibonacci hashing: the high bits
-        at[m] = (unsigned)(h >> 32) & mask;
-        step[m] = (unsigned)(h >> 13) | 1u;  // (odd: the walk meets every entry)
+        coin_place(b, c0[0] + i, c0[1] + j, c0[2] + k, mask, at[m], step[m]);
         old[m] = atomicCAS(&table[at[m]], -1, (int)g);
       }
     }
-    bool hit = false;
+    unsigned found = 0;
 #pragma unroll
     for (int m = 0; m < 8; m++)
-      for (int probe = 1; old[m] != -1 && !hit; probe++) {
-        const double* o = x + 3ll * old[m];  // (both loads under way at once)
-        const int ob = node_blk[old[m]];
-        const double d = fabs(p[0] - o[0]) + fabs(p[1] - o[1]) + fabs(p[2] - o[2]);
-        hit = (old[m] != (int)g && ob == b && d < delta) || probe == kCoinProbes;
-        if (hit) break;
+      for (int probe = 1; old[m] != -1 && !found; probe++) {
+        if (coin_close(x, node_blk, p, (int)g, b, old[m], delta)) found = kCoinClose;
+        else if (probe == kCoinWalk) found = kCoinCrowded;
+        else if (probe % 16 == 0 && *(volatile unsigned*)flag) found = kCoinCrowded;  // (or decided: no more to do)
+        if (found) break;
         at[m] = (at[m] + step[m]) & mask;
         old[m] = atomicCAS(&table[at[m]], -1, (int)g);
       }
-    if (hit) atomicOr(flag, 1u);
+    if (found) atomicOr(flag, found);
+  }
+}
+
+// The crowded gate: every node under its own cell (the table is less than half
+// full), then against the cells its delta-box touches.
+__global__ void k_coin_file(const double* __restrict__ x, const blk_t* __restrict__ node_blk,
+                            const BlockInfo* __restrict__ bi, long long ntot, int* __restrict__ table, unsigned mask,
+                            unsigned* __restrict__ flag) {
+  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ntot;
+       g += (long long)gridDim.x * blockDim.x) {
+    const int b = node_blk[g];
+    const double p[3] = {x[3 * g], x[3 * g + 1], x[3 * g + 2]};
+    const double delta = coin_delta(bi[b]), inv = 1.0 / (kCoinFine * delta);
+    int c[3];
+    for (int k = 0; k < 3; k++) c[k] = (int)floor((p[k] - (double)bi[b].bb_lo[k]) * inv + 0.37);
+    unsigned at, step;
+    coin_place(b, c[0], c[1], c[2], mask, at, step);
+    for (int probe = 1;; probe++) {
+      const int old = atomicCAS(&table[at], -1, (int)g);
+      if (old == -1) break;
+      if (coin_close(x, node_blk, p, (int)g, b, old, delta) || probe == kCoinProbes) {
+        atomicOr(flag, kCoinClose);
+        break;
+      }
+      if (probe % 16 == 0 && (*(volatile unsigned*)flag & kCoinClose)) break;
+      at = (at + step) & mask;
+    }
+  }
+}
+__global__ void k_coin_compare(const double* __restrict__ x, const blk_t* __restrict__ node_blk,
+                               const BlockInfo* __restrict__ bi, long long ntot, const int* __restrict__ table,
+                               unsigned mask, unsigned* __restrict__ flag) {
+  if (*(volatile unsigned*)flag & kCoinClose) return;  // decided (and the table may not be complete)
+  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ntot;
+       g += (long long)gridDim.x * blockDim.x) {
+    const int b = node_blk[g];
+    const double p[3] = {x[3 * g], x[3 * g + 1], x[3 * g + 2]};
+    const double delta = coin_delta(bi[b]), inv = 1.0 / (kCoinFine * delta);
+    constexpr double reach = 0.498;  // delta in cells (1 / 2.01), with room for the rounding; a node's box touches two at most
+    int c0[3], c1[3];
+    for (int k = 0; k < 3; k++) {
+      const double t = (p[k] - (double)bi[b].bb_lo[k]) * inv + 0.37;
+      c0[k] = (int)floor(t - reach);
+      c1[k] = (int)floor(t + reach);
+    }
+    bool close = false;
+    for (int i = c0[0]; i <= c1[0]; i++)
+      for (int j = c0[1]; j <= c1[1]; j++)
+        for (int k = c0[2]; k <= c1[2]; k++) {
+          unsigned at, step;
+          coin_place(b, i, j, k, mask, at, step);
+          for (int old = table[at]; old != -1 && !close; old = table[at = (at + step) & mask])
+            close = coin_close(x, node_blk, p, (int)g, b, old, delta);
+        }
+    if (close) atomicOr(flag, kCoinClose);
   }
 }
 
