@@ -133,3 +133,24 @@ def test_coincidence_gate_of_graded_blocks(inner, gap, oracle_lib):
         ms = _preprocess_ms(t)
         t.delete()
         assert ms < 6 * plain_ms, (ms, plain_ms)
+
+
+@pytest.mark.parametrize("octaves", [40, 180, 400])
+def test_merge_of_points_across_many_octaves(octaves, oracle_lib):
+    """Query points at distances 1, 1/2, 1/4 ... from a plane and thirty
+    coincident ones beyond the last: a split halves a box, so they are apart
+    only after as many levels as there are octaves.  At most 33 are farther
+    apart than TOL and each of the merge's 128 levels takes one away, so all
+    but 162 are merged, also where there are more octaves than levels."""
+    base = cases.config0(2, nbg=13, nr=9, nt=11, nphi=21, perturb=0.0)
+    bg = base.blocks[0]
+    d = np.concatenate([2.0 ** -np.arange(octaves), np.full(30, 2.0 ** -octaves)])
+    extra = np.stack([d, np.full(len(d), 0.8), np.full(len(d), 0.3)], 1)
+    system = cases.System([cases.Block(bg.tag, np.concatenate([bg.x, extra]), bg.cells, bg.wbc, bg.obc),
+                           *base.blocks[1:]])
+    ref = run_system(oracle_lib, system)
+    t = _connected(system)
+    assert tb.stats(t.lib)["nmerged"] >= max(29, len(d) - 162), tb.stats(t.lib)
+    for b in system.blocks:
+        assert np.array_equal(ref["iblank"][b.tag], t.iblank(b.tag))
+    t.delete()

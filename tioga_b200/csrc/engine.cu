@@ -1744,7 +1744,8 @@ int Engine::dedup_merge(const DedupQueries& Qd, const std::vector<int>& qoff) {
     k_dedup_octant<<<grid_for(n, kT), kT, 0, stream_>>>(n, dd_seg_.p, dd_perm_.p, dd_x_.p, dd_S_.p, dd_oct_.p, nseg);
     TB_LAUNCHED("k_dedup_octant");
     k_dedup_split<<<grid_for((long long)nseg_cap, 128, 148), 128, 0, stream_>>>(
-        dd_S_.p, dd_T_.p, dd_leaves_.p, dd_cnt_.p, nseg, dd_cnt_.p + kDedupSegs + level + 1);
+        dd_S_.p, dd_T_.p, dd_leaves_.p, dd_cnt_.p, nseg, dd_cnt_.p + kDedupSegs + level + 1,
+        level + 1 == kDedupLevels);
     TB_LAUNCHED("k_dedup_split");
     k_dedup_scatter<<<grid_for(n, kT), kT, 0, stream_>>>(n, dd_seg_.p, dd_perm_.p, dd_x_.p, dd_S_.p, dd_T_.p,
                                                          dd_oct_.p, nseg, dd_seg2_.p, dd_perm2_.p, dd_member_.p);

@@ -242,7 +242,8 @@ __global__ void k_dedup_gather(const int* refq, long long n, const int* qnode, c
                                int* itag, int* perm, int* member, int* seg, int* gpos_of);
 __global__ void k_dedup_octant(long long n, const int* seg, const int* perm, const double* xg, DedupSeg* S,
                                unsigned char* oct, const int* nseg);
-__global__ void k_dedup_split(DedupSeg* S, DedupSeg* T, int4* leaves, int* cnt, const int* nseg, int* nnext);
+__global__ void k_dedup_split(DedupSeg* S, DedupSeg* T, int4* leaves, int* cnt, const int* nseg, int* nnext,
+                              int last);
 __global__ void k_dedup_scatter(long long n, const int* seg, const int* perm, const double* xg, DedupSeg* S,
                                 DedupSeg* T, const unsigned char* oct, const int* nseg, int* seg2, int* perm2,
                                 int* member);

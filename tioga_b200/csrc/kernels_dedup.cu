@@ -377,9 +377,10 @@ __global__ void k_dedup_octant(long long n, const int* __restrict__ seg, const i
 
 // every active subset's children: the next level's subsets, or leaves (child
 // of octant o: first position base[o], next-level subset child[o] or -1).  All
-// points in one octant: the subset itself is a leaf (icheck).
+// points in one octant: the subset itself is a leaf (icheck).  On the last level
+// every child is a leaf.
 __global__ void k_dedup_split(DedupSeg* __restrict__ S, DedupSeg* __restrict__ T, int4* __restrict__ leaves,
-                              int* __restrict__ cnt, const int* __restrict__ nseg, int* __restrict__ nnext) {
+                              int* __restrict__ cnt, const int* __restrict__ nseg, int* __restrict__ nnext, int last) {
   const int ns = *nseg;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
     DedupSeg& g = S[s];
@@ -392,7 +393,7 @@ __global__ void k_dedup_split(DedupSeg* __restrict__ S, DedupSeg* __restrict__ T
       g.base[o] = at;
       g.child[o] = -1;
       if (m > 0 && !one) {
-        if (m > kDedupLeaf) {
+        if (m > kDedupLeaf && !last) {
           const int t = atomicAdd(nnext, 1);
           T[t].start = at;
           T[t].len = m;
