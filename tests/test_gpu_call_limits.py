@@ -154,3 +154,68 @@ def test_merge_of_points_across_many_octaves(octaves, oracle_lib):
     for b in system.blocks:
         assert np.array_equal(ref["iblank"][b.tag], t.iblank(b.tag))
     t.delete()
+
+
+def test_fp64_walks_far_from_the_origin(oracle_lib):
+    """The FP64 form on a mesh moved by 2^20 with cells of about 1/128 (every
+    coordinate exact in both places): the oracle's result there, and walks as
+    short as at the origin."""
+    base = cases.config0(3, nbg=41, nr=13, nt=25, nphi=49, perturb=0.02)
+    ms = {}
+    for offset in (0.0, 2.0 ** 20):
+        system = cases.System([cases.Block(b.tag, np.round(b.x / 26.0 * 2.0 ** 26) / 2.0 ** 26 + offset, b.cells,
+                                           b.wbc, b.obc) for b in base.blocks])
+        ref = run_system(oracle_lib, system)
+        t = TiogaLibrary(tb.library_path())
+        tb.extras(t.lib)
+        t.init()
+        t.register_system(system)
+        tb.set_int(t.lib, "tioga_b200_set_precision_", 0)
+        t.preprocess_grids()
+        walk = []
+        for _ in range(5):
+            t.performconnectivity()
+            assert t.lib.tioga_b200_last_error() == 0
+            walk.append(tb.timing(t.lib)["search_traverse"])
+        ms[offset] = min(walk)
+        for b in system.blocks:
+            assert np.array_equal(ref["iblank"][b.tag], t.iblank(b.tag))
+            for a, c in zip(ref["donors"][b.tag], t.getdonorinfo(b.tag)):
+                assert np.array_equal(a, c)
+        t.delete()
+    assert ms[2.0 ** 20] < 4 * ms[0.0], ms
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_high_order_search_in_another_form_than_the_last_call(form):
+    """The precision changed between the connectivity call and the high-order
+    one: the same point donors as with one precision throughout."""
+    system, ho = cases.small_config4()
+    got = []
+    for forms in ((form, form), (1 - form, form)):
+        t = TiogaLibrary(tb.library_path())
+        tb.extras(t.lib)
+        t.init()
+        t.register_system(system)
+        for b, h in zip(system.blocks, ho):
+            x = np.ascontiguousarray(h.xdof)
+            t._keep.append(x)
+            t.lib.tioga_b200_set_highorder_lagrange_(C.byref(C.c_int(b.tag)), C.byref(C.c_int(h.p)),
+                                                     x.ctypes.data_as(C.c_void_p))
+        t.preprocess_grids()
+        tb.set_int(t.lib, "tioga_b200_set_precision_", forms[0])
+        t.performconnectivity()
+        tb.set_int(t.lib, "tioga_b200_set_precision_", forms[1])
+        t.lib.tioga_performconnectivity_highorder_()
+        assert t.lib.tioga_b200_last_error() == 0
+        points = []
+        for b in system.blocks:
+            n = t.lib.tioga_b200_pointdonors_(C.byref(C.c_int(b.tag)), None, None)
+            rec = np.zeros((max(n, 1), 4), np.int32)
+            t.lib.tioga_b200_pointdonors_(C.byref(C.c_int(b.tag)), rec.ctypes.data_as(C.c_void_p), None)
+            points.append(rec[:n])
+        got.append(points)
+        t.delete()
+    assert sum(len(p) for p in got[0]) > 0
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)

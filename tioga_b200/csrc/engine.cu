@@ -601,9 +601,9 @@ int Engine::upload_chunked() {
     }
     const long long l0 = h_up_leaf_off_[k], nl = h_up_leaf_off_[k + 1] - l0;
     if (nl > 0) {
-      launch_cell_boxes(1, mb, (int)grid_for(nl * kMaxLeafCells, 256, 148 * mb), stream_, x_.p, xf_.p, conn8_.p,
-                        cell_nv_.p, leaves_.p, up_leaf_ids_.p + l0, nullptr, nullptr, nl, cbox_.p, nullptr, tnode_.p,
-                        lbox_.p);
+      launch_cell_boxes(1, mb, (int)grid_for(nl * kMaxLeafCells, 256, 148 * mb), stream_, x_.p, d_bi_.p, xf_.p,
+                        conn8_.p, cell_nv_.p, leaves_.p, up_leaf_ids_.p + l0, nullptr, nullptr, nl, cbox_.p, nullptr,
+                        tnode_.p, lbox_.p);
       TB_LAUNCHED("k_cell_boxes");
     }
   }
@@ -618,6 +618,7 @@ int Engine::upload_chunked() {
   coords_on_device_ = true;
   gate_valid_ = false;  // the caller may have moved the nodes any way
   boxes_ready_ = true;
+  boxes_form_ = 1;
   groups_culled_ = false;
   groups_stale_ = true;
   tiles_ready_ = h_up_tile_off_.size() == h_up_leaf_off_.size();
@@ -1249,6 +1250,7 @@ int Engine::run_pairs_and_refit() {
     }
   }
   if (boxes) {  // (the chunked upload has set these)
+    boxes_form_ = fp64 ? 0 : 1;
     groups_culled_ = cull;
     groups_stale_ = !cull;
   }
@@ -1316,9 +1318,9 @@ int Engine::run_pairs_and_refit() {
   const size_t smem = (size_t)maxnp * (6 * sizeof(unsigned long long) + sizeof(PairCull) + 6 * sizeof(int));
   const int mb = tune_.cell_box_per_sm;
   if (!boxes_ready_) {  // else made during the chunked upload
-    launch_cell_boxes(fp64 ? 0 : 1, mb, (int)grid_for(nleaf_total_ * kMaxLeafCells, 256, 148 * mb), stream_, x_.p, xf_.p, conn8_.p,
-                      cell_nv_.p, leaves_.p, nullptr, cull ? grp_act_.p : nullptr, nact_.p, nleaf_total_, cbox_.p, cbox64_.p,
-                      tnode_.p, lbox_.p);
+    launch_cell_boxes(fp64 ? 0 : 1, mb, (int)grid_for(nleaf_total_ * kMaxLeafCells, 256, 148 * mb), stream_, x_.p,
+                      d_bi_.p, xf_.p, conn8_.p, cell_nv_.p, leaves_.p, nullptr, cull ? grp_act_.p : nullptr, nact_.p,
+                      nleaf_total_, cbox_.p, cbox64_.p, tnode_.p, lbox_.p);
     TB_LAUNCHED("k_cell_boxes");
   }
   TB_CUDA(cudaEventRecord(hev_[0], stream_));  // the hole maps may start
@@ -1351,9 +1353,10 @@ int Engine::launch_refit(cudaStream_t st) {
   return 0;
 }
 
-// (the pairs come out as they are: the boxes are what this is for)
+// (the pairs come out as they are: the boxes are what this is for, those of the
+// form the search will walk)
 int Engine::all_cell_boxes() {
-  if (!groups_culled_) return 0;
+  if (!groups_culled_ && boxes_form_ == (precision_ == 0 ? 0 : 1)) return 0;
   fetch_timing();  // the call's own times: the events are recorded anew below
   boxes_ready_ = tiles_ready_ = false;
   TB_TRY(run_pairs_and_refit());

@@ -102,10 +102,10 @@ __global__ void k_pairs(const BlockInfo* bi, int nb, const int2* cand, int ncand
                         int* pfirst, unsigned long long* acc, int* ext, int* blk_bnd);
 __global__ void k_pair_finish(const BlockInfo* bi, PairInfo* pairs, int npairs,
                               const unsigned long long* acc);
-void launch_cell_boxes(int form, int minb, int grid, cudaStream_t st, const double* x, const float4* xf,
-                       const int* conn8, const unsigned char* cell_nv, const int4* leaves, const int* ids,
-                       const int* act, const unsigned* nact, long long nleaf, float2* cbox, double* cbox64,
-                       float4* tnode, float4* lbox);
+void launch_cell_boxes(int form, int minb, int grid, cudaStream_t st, const double* x, const BlockInfo* bi,
+                       const float4* xf, const int* conn8, const unsigned char* cell_nv, const int4* leaves,
+                       const int* ids, const int* act, const unsigned* nact, long long nleaf, float2* cbox,
+                       double* cbox64, float4* tnode, float4* lbox);
 __global__ void k_leaf_chunk(const int4* leaves, long long nleaf, const int* conn8, const unsigned char* cell_nv,
                              int chunk, int* key, int* id);
 __global__ void k_round_nodes(const double* x, long long lo, long long hi, float4* xf, unsigned* err);

@@ -591,6 +591,15 @@ __global__ void k_pair_finish(const BlockInfo* __restrict__ bi, PairInfo* __rest
 // bounding-volume tree: cell boxes in Morton order, leaves of up to
 // kMaxLeafCells cells, implicit complete 4-ary tree (heap order) per block
 // ===========================================================================
+// The FP64 form's tree holds its FP32 boxes relative to a point inside the
+// block, so what they are rounded to goes with the block's size and not with
+// its distance from the origin: with cells of 1/128 at 2^20 every walk visited
+// thousands of cells (22 k queries 10.85 ms, 0.07 ms with it and at the
+// origin; with FP64 boxes in the tree 0.22 ms in both places).  A box holds a point after the subtraction if it did before, as
+// rounding keeps the order.
+__device__ __forceinline__ double tree_origin(const BlockInfo& B, int k) {
+  return isfinite(B.obb.xc[k]) ? B.obb.xc[k] : 0.0;
+}
 __device__ __forceinline__ float f_rd(double v) { return __double2float_rd(v); }
 __device__ __forceinline__ float f_ru(double v) { return __double2float_ru(v); }
 
@@ -916,6 +925,7 @@ __device__ __forceinline__ void cell_box_load(const float2* __restrict__ cbox, l
 // three take 167 us and one code path.)
 template <int MINB, int FORM>
 __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restrict__ x,
+                                                          const BlockInfo* __restrict__ bi,
                                                           const float4* __restrict__ xf,
                                                           const int* __restrict__ conn8,
                                                           const unsigned char* __restrict__ cell_nv,
@@ -940,6 +950,7 @@ __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restri
     const bool valid = leaf_ok && lane % LC < L.y;
     const long long c = (long long)L.x + lane % LC;
     float f[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    float r[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};  // FORM 0: the tree's
     if (valid) {
       const int nv = cell_nv[c];
       const int4 c0 = *reinterpret_cast<const int4*>(conn8 + 8 * c);
@@ -963,6 +974,9 @@ __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restri
         for (int k = 0; k < 3; k++) {
           f[k] = f_rd(lo[k]);
           f[k + 3] = f_ru(hi[k]);
+          const double o = tree_origin(bi[L.w], k);
+          r[k] = f_rd(lo[k] - o);
+          r[k + 3] = f_ru(hi[k] - o);
         }
       } else {
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -985,11 +999,16 @@ __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restri
       for (int k = 0; k < 3; k++) {
         f[k] = fminf(f[k], __shfl_xor_sync(0xffffffffu, f[k], o));
         f[k + 3] = fmaxf(f[k + 3], __shfl_xor_sync(0xffffffffu, f[k + 3], o));
+        if (FORM == 0) {
+          r[k] = fminf(r[k], __shfl_xor_sync(0xffffffffu, r[k], o));
+          r[k + 3] = fmaxf(r[k + 3], __shfl_xor_sync(0xffffffffu, r[k + 3], o));
+        }
       }
     if (leaf_ok && lane % LC == 0) {
       const long long sl = L.z;
-      tnode[2 * sl] = make_float4(f[0], f[1], f[2], f[3]);
-      *reinterpret_cast<float2*>(&tnode[2 * sl + 1]) = make_float2(f[4], f[5]);  // keep the link
+      const float* t = FORM == 0 ? r : f;
+      tnode[2 * sl] = make_float4(t[0], t[1], t[2], t[3]);
+      *reinterpret_cast<float2*>(&tnode[2 * sl + 1]) = make_float2(t[4], t[5]);  // keep the link
       lbox[2 * leaf] = make_float4(f[0], f[1], f[2], f[3]);
       lbox[2 * leaf + 1] = make_float4(f[4], f[5], __int_as_float(L.w), 0.f);
     }
@@ -1186,12 +1205,12 @@ static void set_smem(K kern, size_t smem) {
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
-void launch_cell_boxes(int form, int minb, int grid, cudaStream_t st, const double* x, const float4* xf,
-                       const int* conn8, const unsigned char* cell_nv, const int4* leaves, const int* ids,
-                       const int* act, const unsigned* nact, long long nleaf, float2* cbox, double* cbox64,
-                       float4* tnode, float4* lbox) {
+void launch_cell_boxes(int form, int minb, int grid, cudaStream_t st, const double* x, const BlockInfo* bi,
+                       const float4* xf, const int* conn8, const unsigned char* cell_nv, const int4* leaves,
+                       const int* ids, const int* act, const unsigned* nact, long long nleaf, float2* cbox,
+                       double* cbox64, float4* tnode, float4* lbox) {
 #define TB_CB(MB, F)                                                                                            \
-  k_cell_boxes<MB, F><<<grid, 256, 0, st>>>(x, xf, conn8, cell_nv, leaves, ids, act, nact, nleaf, cbox, cbox64, \
+  k_cell_boxes<MB, F><<<grid, 256, 0, st>>>(x, bi, xf, conn8, cell_nv, leaves, ids, act, nact, nleaf, cbox, cbox64, \
                                             tnode, lbox)
   if (form == 0) TB_CB(3, 0);  // (its FP64 vertices take the registers of fewer CTAs)
   else if (minb <= 4) TB_CB(4, 1);
@@ -1821,8 +1840,9 @@ __global__ void __launch_bounds__(kWalkThreads) k_traverse(
     for (int k = 0; k < 3; k++) {
       const float p32 = (float)p[k];
       const float e = fabsf(p32) * 9.6e-7f + 2e-9f;
-      plo[k] = FORM == 0 ? f_rd(p[k] - 2 * kTol) : p32 - e;
-      phi[k] = FORM == 0 ? f_ru(p[k] + 2 * kTol) : p32 + e;
+      const double o = FORM == 0 ? tree_origin(bi[qdon[q]], k) : 0.0;
+      plo[k] = FORM == 0 ? f_rd((p[k] - 2 * kTol) - o) : p32 - e;
+      phi[k] = FORM == 0 ? f_ru((p[k] + 2 * kTol) - o) : p32 + e;
     }
     // cells [c0, c0 + nc) of a hit leaf (1 <= nc <= kMaxLeafCells).  FP32
     // boxes: four cells at a time, every slot reading a cell of the leaf (the
@@ -1953,10 +1973,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_traverse_quad(
   for (long long q0 = ((long long)blockIdx.x * kWalkThreads + (t & ~31)) / 4; q0 < nq; q0 += nqs) {
     const long long q = q0 + (lane >> 2);
     const bool mine = q < nq && sub == 0;  // writes the query's results
-    int n = 0, g = 0, root = -1;
+    int n = 0, g = 0, d = 0, root = -1;
     if (q < nq) {
       g = qnode[q];
-      const int d = qdon[q];
+      d = qdon[q];
       // (else k_uhex_search's, or merged into another)
       if (!(skip_uhex && bi[d].uhex) && !(q_rep && q_rep[q] != q)) root = bi[d].root;
     }
@@ -1974,8 +1994,9 @@ __global__ void __launch_bounds__(kWalkThreads) k_traverse_quad(
       p[k] = x[3 * (long long)g + k];
       const float p32 = (float)p[k];
       const float e = fabsf(p32) * 9.6e-7f + 2e-9f;
-      plo[k] = FORM == 0 ? f_rd(p[k] - 2 * kTol) : p32 - e;
-      phi[k] = FORM == 0 ? f_ru(p[k] + 2 * kTol) : p32 + e;
+      const double o = FORM == 0 ? tree_origin(bi[d], k) : 0.0;
+      plo[k] = FORM == 0 ? f_rd((p[k] - 2 * kTol) - o) : p32 - e;
+      phi[k] = FORM == 0 ? f_ru((p[k] + 2 * kTol) - o) : p32 + e;
     }
     // cells [c0, c0 + nc) of a hit leaf (nc <= kMaxLeafCells; 0: none), by all
     // lanes of the warp together; hits are added in cell order
