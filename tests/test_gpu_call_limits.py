@@ -219,3 +219,66 @@ def test_high_order_search_in_another_form_than_the_last_call(form):
     assert sum(len(p) for p in got[0]) > 0
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("where", ["pinned", "mixed"])
+def test_device_arrays_that_only_copies_reach(where, oracle_lib):
+    """Page-locked host memory given as a device iblank array, for all blocks
+    and for one beside a device array: written by copies, as another GPU's
+    memory would be."""
+    import torch
+    system = cases.config1(4, nbg=17, nshell=2, nr=7, nt=7, nphi=13, split_layers=2)
+    ref = run_system(oracle_lib, system)
+    t = TiogaLibrary(tb.library_path())
+    tb.extras(t.lib)
+    t.init()
+    t.register_system(system)
+    ibl = []
+    for i, b in enumerate(system.blocks):
+        here = where == "mixed" and i != 1
+        a = torch.full((b.nnodes,), -7, dtype=torch.int32, device="cuda" if here else "cpu", pin_memory=not here)
+        ibl.append(a)
+        t.lib.tioga_b200_registeriblank_device_(C.byref(C.c_int(b.tag)), C.c_void_p(a.data_ptr()))
+    torch.cuda.synchronize()
+    t.preprocess_grids()
+    assert t.lib.tioga_b200_last_error() == 0
+    for a in ibl:
+        assert (a == 1).all()
+    t.performconnectivity()
+    assert t.lib.tioga_b200_last_error() == 0
+    for b, a in zip(system.blocks, ibl):
+        assert np.array_equal(ref["iblank"][b.tag], a.cpu().numpy())
+    t.delete()
+
+
+def test_high_order_fields_that_only_copies_reach():
+    """Device solutions of the high-order update in page-locked host memory
+    for one block: the same values as with both on the device."""
+    import torch
+    system, ho = cases.small_config4()
+    q0 = [np.ascontiguousarray(q, dtype=np.float64).reshape(-1) for q in cases.dof_fields(ho, 2, seed=3)]
+    got = []
+    for pinned in (False, True):
+        t = TiogaLibrary(tb.library_path())
+        tb.extras(t.lib)
+        t.init()
+        t.register_system(system)
+        for b, h in zip(system.blocks, ho):
+            x = np.ascontiguousarray(h.xdof)
+            t._keep.append(x)
+            t.lib.tioga_b200_set_highorder_lagrange_(C.byref(C.c_int(b.tag)), C.byref(C.c_int(h.p)),
+                                                     x.ctypes.data_as(C.c_void_p))
+        t.preprocess_grids()
+        t.performconnectivity()
+        t.lib.tioga_performconnectivity_highorder_()
+        q = [torch.from_numpy(a.copy()) for a in q0]
+        q = [a.pin_memory() if pinned and i == 1 else a.cuda() for i, a in enumerate(q)]
+        for b, a in zip(system.blocks, q):
+            t.lib.tioga_b200_registersolution_device_(C.byref(C.c_int(b.tag)), C.c_void_p(a.data_ptr()))
+        t.dataupdate_mb(2, "row")
+        assert t.lib.tioga_b200_last_error() == 0
+        got.append([a.cpu().numpy() for a in q])
+        t.delete()
+    assert any((a != b).any() for a, b in zip(got[0], q0))
+    for a, b in zip(*got):
+        assert np.array_equal(a.view(np.int64), b.view(np.int64))

@@ -22,6 +22,13 @@ def test_buffers_go_back_after_the_work_that_reads_them(tmp_path):
     _run(tmp_path, "devmem_check.cc", "g++", "-I", os.path.join(cuda, "include"))
 
 
+def test_kernels_work_on_arrays_of_their_own_device_only(tmp_path):
+    """A caller's array that a kernel may not reach (another GPU's, host or
+    misaligned memory) is left to copies."""
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    _run(tmp_path, "reach_check.cc", "g++", "-I", os.path.join(cuda, "include"))
+
+
 def test_donor_slots_refuse_indices_outside_their_arrays(tmp_path):
     """Both kernels that fill the donor slots take their places from here."""
     _run(tmp_path, "donor_slots_check.cu", os.environ.get("NVCC", "nvcc"))

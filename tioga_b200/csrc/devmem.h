@@ -12,6 +12,22 @@
 
 namespace tb {
 
+// Whether a kernel on device `dev` may work on a caller's array at p: device
+// memory of that device, aligned for its elements.  Anything else (another
+// GPU's memory, which needs peer access, managed or host memory) is left to
+// copies, which reach it without.
+inline bool kernel_reaches(const cudaPointerAttributes& a, int dev, const void* p, size_t align) {
+  return a.type == cudaMemoryTypeDevice && a.device == dev && reinterpret_cast<uintptr_t>(p) % align == 0;
+}
+inline bool kernel_reaches(const void* p, int dev, size_t align) {
+  cudaPointerAttributes a = {};
+  if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return kernel_reaches(a, dev, p, align);
+}
+
 // Device bytes of the engine whose calls this thread is running (the
 // serving form's admission accounting); null: not counted.
 extern thread_local long long* g_dbuf_account;

@@ -27,6 +27,7 @@ int sync_check() {
 }
 
 Engine::Engine() {
+  cudaGetDevice(&device_);
   // The side stream's kernels are wide (the hole-map fill fills the device with
   // CTAs) and nothing waits for them before the donor phase, so the main
   // stream goes first wherever a CTA slot frees up.
@@ -195,6 +196,7 @@ int Engine::register_iblank_device(int tag, int* d_ibl) {
   int ib = find_tag(tag);
   if (ib < 0) return -1;
   hb_[ib].dibl = d_ibl;
+  hb_[ib].dibl_here = kernel_reaches(d_ibl, device_, sizeof(int));
   return 0;
 }
 
@@ -2054,16 +2056,17 @@ int Engine::run_celliblank() {
 
 // The node iblanks into the callers' device arrays, one launch over all
 // blocks (a copy per block took 4 us each: 270 us for a batch of 63 blocks),
-// and with `host` into their host arrays.
+// a copy where a kernel may not write, and with `host` into their host arrays.
 int Engine::write_iblanks(bool host) {
   bool device = false;
-  for (const HostBlock& H : hb_) device = device || H.dibl;
+  for (const HostBlock& H : hb_) device = device || (H.dibl && H.dibl_here);
   if (device && ntot_ > 0) {
     std::vector<int*> ptr(hb_.size());
     for (size_t b = 0; b < hb_.size(); b++)
-      ptr[b] = hb_[b].dibl ? reinterpret_cast<int*>(reinterpret_cast<uintptr_t>(hb_[b].dibl) -
-                                                    sizeof(int) * (uintptr_t)bi_[b].node_off)
-                           : nullptr;
+      ptr[b] = hb_[b].dibl && hb_[b].dibl_here
+                   ? reinterpret_cast<int*>(reinterpret_cast<uintptr_t>(hb_[b].dibl) -
+                                            sizeof(int) * (uintptr_t)bi_[b].node_off)
+                   : nullptr;
     if (ptr != h_iblptr_ || !d_iblptr_.p) {
       TB_CUDA(d_iblptr_.ensure(ptr.size()));
       TB_CUDA(cudaMemcpyAsync(d_iblptr_.p, ptr.data(), ptr.size() * sizeof(int*), cudaMemcpyHostToDevice, stream_));
@@ -2072,10 +2075,12 @@ int Engine::write_iblanks(bool host) {
     k_write_iblanks<<<grid_for(ntot_, kT), kT, 0, stream_>>>(iblank_.p, node_blk_.p, ntot_, d_iblptr_.p);
     TB_LAUNCHED("k_write_iblanks");
   }
-  for (size_t b = 0; b < hb_.size() && host; b++)
-    if (!hb_[b].dibl)
-      TB_CUDA(cudaMemcpyAsync(hb_[b].hibl, iblank_.p + bi_[b].node_off, hb_[b].nnodes * sizeof(int),
-                              cudaMemcpyDeviceToHost, stream_));
+  for (size_t b = 0; b < hb_.size(); b++) {
+    const HostBlock& H = hb_[b];
+    if (H.dibl ? H.dibl_here : !host) continue;
+    TB_CUDA(cudaMemcpyAsync(H.dibl ? H.dibl : H.hibl, iblank_.p + bi_[b].node_off, H.nnodes * sizeof(int),
+                            H.dibl ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, stream_));
+  }
   return 0;
 }
 

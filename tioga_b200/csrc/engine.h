@@ -227,6 +227,7 @@ struct HostBlock {
   double* hq = nullptr;          // registered host solution
   double* dq = nullptr;          // registered device solution
   int* dibl = nullptr;           // caller's device iblank array (optional)
+  bool dibl_here = false;        // and whether a kernel may write it (kernel_reaches)
   const uint64_t* cell_gid = nullptr;  // caller's cell global ids (registerGridData's cell_gid)
 };
 
@@ -379,6 +380,7 @@ class Engine {
   int last_error() const { return last_error_; }
 
  private:
+  int device_ = 0;  // the instance's device
   std::shared_ptr<DevPool> dev_pool_;
   // declared before every buffer, so it outlives them: the stream that
   // stream-ordered buffers are freed on

@@ -530,15 +530,20 @@ int Engine::dataupdate_highorder(int nvar, int interptype) {
   }
   std::vector<long long> qo(nb + 1, 0);
   for (int b = 0; b < nb; b++) qo[b + 1] = qo[b] + (long long)hb_[b].ncells * ho_[b].npts * nvar;
-  // host fields go through a copy; device fields are read and written in
-  // place (every value is gathered into ho_qtmp_ before the first is written)
+  // device fields are read and written in place (every value is gathered into
+  // ho_qtmp_ before the first is written); host fields, and arrays that a
+  // kernel may not work on, go through a copy
   std::vector<double*> qptr(nb);
-  if (host) TB_CUDA(ho_q_.ensure(std::max(1ll, qo[nb])));
+  std::vector<char> copied(nb);
   for (int b = 0; b < nb; b++) {
-    qptr[b] = host ? ho_q_.p + qo[b] : hb_[b].dq;
-    if (host)
-      TB_CUDA(cudaMemcpyAsync(qptr[b], hb_[b].hq, (qo[b + 1] - qo[b]) * sizeof(double), cudaMemcpyHostToDevice,
-                              stream_));
+    copied[b] = host || !kernel_reaches(hb_[b].dq, device_, sizeof(double));
+    if (copied[b]) TB_CUDA(ho_q_.ensure(std::max(1ll, qo[nb])));
+  }
+  for (int b = 0; b < nb; b++) {
+    qptr[b] = copied[b] ? ho_q_.p + qo[b] : hb_[b].dq;
+    if (copied[b])
+      TB_CUDA(cudaMemcpyAsync(qptr[b], host ? hb_[b].hq : hb_[b].dq, (qo[b + 1] - qo[b]) * sizeof(double),
+                              host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, stream_));
   }
   TB_TRY(upload_qptr(qptr));
   const long long ntp = ho_pt_off_[nb];
@@ -568,10 +573,11 @@ int Engine::dataupdate_highorder(int nvar, int interptype) {
                                                                    d_qptr_.p);
     TB_LAUNCHED("k_ho_scatter");
   }
-  // host fields back to the caller, and the cell iblanks the orphan rule changed
-  for (int b = 0; b < nb && host; b++)
-    TB_CUDA(cudaMemcpyAsync(hb_[b].hq, qptr[b], (qo[b + 1] - qo[b]) * sizeof(double), cudaMemcpyDeviceToHost,
-                            stream_));
+  // copied fields back to the caller, and the cell iblanks the orphan rule changed
+  for (int b = 0; b < nb; b++)
+    if (copied[b])
+      TB_CUDA(cudaMemcpyAsync(host ? hb_[b].hq : hb_[b].dq, qptr[b], (qo[b + 1] - qo[b]) * sizeof(double),
+                              host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, stream_));
   unsigned long long orphans = 0;
   TB_CUDA(cudaMemcpyAsync(&orphans, counters_.p + 8, sizeof(orphans), cudaMemcpyDeviceToHost, stream_));
   TB_CUDA(cudaStreamSynchronize(stream_));
