@@ -153,6 +153,7 @@ int main() {
   auto pool = std::make_shared<tb::DevPool>();
   pool->users = {main_st, side};
   tb::g_dbuf_dev = pool;
+  expect(pools == 0 && streams.size() == 2, "the pool is made before there is a buffer");
   {
     // buffers that grow while kernels of either stream still read them
     tb::DBuf<char> a, b, c;
