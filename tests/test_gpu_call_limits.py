@@ -282,3 +282,29 @@ def test_high_order_fields_that_only_copies_reach():
     assert any((a != b).any() for a, b in zip(got[0], q0))
     for a, b in zip(*got):
         assert np.array_equal(a.view(np.int64), b.view(np.int64))
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "split"])
+def test_batch_past_the_four_lane_walk(precision, oracle_lib):
+    """A batch that is shown to have the million queries from which a walk
+    has one lane, against the oracle, system by system."""
+    two = [cases.config0(s, nbg=49, nr=17, nt=25, nphi=49, perturb=0.05) for s in (1, 2)]
+    refs = [run_system(oracle_lib, s) for s in two]
+    copies = [cases.System([cases.Block(b.tag, b.x.copy(), b.cells, b.wbc, b.obc) for b in two[k % 2].blocks])
+              for k in range(50)]
+    t = TiogaLibrary(tb.library_path())
+    tb.extras(t.lib)
+    t.init()
+    t.register_batch(copies)
+    tb.set_int(t.lib, "tioga_b200_set_precision_", precision)
+    t.preprocess_grids()
+    t.performconnectivity()
+    assert t.lib.tioga_b200_last_error() == 0
+    assert tb.stats(t.lib)["nquery"] >= 1 << 20, tb.stats(t.lib)
+    for k, system in enumerate(copies):
+        t.select_system(k)
+        got = {"iblank": {b.tag: t.blocks[(k, b.tag)]["iblank"].copy() for b in system.blocks},
+               "donors": {b.tag: t.getdonorinfo(b.tag) for b in system.blocks}, "q": {}}
+        problems = diff_runs(system, refs[k % 2], got)
+        assert not problems, "\n".join(problems)
+    t.delete()
