@@ -308,3 +308,35 @@ def test_batch_past_the_four_lane_walk(precision, oracle_lib):
         problems = diff_runs(system, refs[k % 2], got)
         assert not problems, "\n".join(problems)
     t.delete()
+
+
+@pytest.mark.parametrize("side", ["device", "host"])
+def test_update_after_a_refused_connectivity_call(side, oracle_lib):
+    """A connectivity call refused for a coordinate that is not finite leaves
+    the interpolation of the one before: an update then is the oracle's, and
+    so is the next call on good coordinates."""
+    import torch
+    system = cases.small_config1(2)
+    q0 = cases.fields(system, nvar=3, seed=5)
+    ref = run_system(oracle_lib, system, q_blocks=q0, nvar=3)
+    t = _connected(system)
+    for again in (False, True):
+        x = t.blocks[system.blocks[1].tag]["x"]
+        good = x[7]
+        if not again:
+            x[7] = np.nan
+        t.performconnectivity()
+        assert (t.lib.tioga_b200_last_error() != 0) == (not again)
+        x[7] = good
+        q = [torch.from_numpy(a.copy()).to("cuda" if side == "device" else "cpu") for a in q0]
+        for b, a in zip(system.blocks, q):
+            tag = C.byref(C.c_int(b.tag))
+            if side == "device":
+                t.lib.tioga_b200_registersolution_device_(tag, C.c_void_p(a.data_ptr()))
+            else:
+                t.lib.tioga_registersolution_(tag, C.c_void_p(a.data_ptr()))
+        t.dataupdate_mb(3, "row")
+        assert t.lib.tioga_b200_last_error() == 0
+        for b, a in zip(system.blocks, q):
+            assert np.array_equal(a.cpu().numpy().view(np.int64), ref["q"][b.tag].view(np.int64))
+    t.delete()

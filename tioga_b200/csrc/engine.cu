@@ -300,8 +300,8 @@ int Engine::upload_topology() {
   counters_.p = call_words_.p;
   err_.p = reinterpret_cast<unsigned*>(call_words_.p + 16);
   scount_.p = err_.p + 2;
-  rcount_.p = reinterpret_cast<int*>(call_words_.p + 18);
-  nact_.p = reinterpret_cast<unsigned*>(call_words_.p + 19);
+  nact_.p = reinterpret_cast<unsigned*>(call_words_.p + 18);
+  rcount_.p = reinterpret_cast<int*>(call_words_.p + 19);
   TB_CUDA(h_rb_.ensure(1024));
   TB_CUDA(cudaMemsetAsync(wallf_.p, 0, ntot_, stream_));
   TB_CUDA(cudaMemsetAsync(obcf_.p, 0, ntot_, stream_));
@@ -1824,7 +1824,7 @@ int Engine::run_donors() {
     TB_LAUNCHED("k_classify_tiles");
   }
   // nfringe layers around the holes, then the layers' nodes become mandatory
-  k_front_init<<<1, 1, 0, stream_>>>(dcnt_.p);
+  k_front_init<<<1, 1, 0, stream_>>>(dcnt_.p, rcount_.p);
   TB_LAUNCHED("k_front_init");
   int maxfr = 0;
   for (auto& B : bi_) maxfr = std::max(maxfr, B.nfringe);
@@ -2200,8 +2200,9 @@ int Engine::connectivity() {
   interps_fetched_ = false;
   update_lists_ = false;
   TB_CUDA(cudaEventRecord(ev_[0], stream_));
-  // this call's counters and device errors only
-  TB_CUDA(cudaMemsetAsync(call_words_.p, 0, kCallWords * sizeof(unsigned long long), stream_));
+  // this call's counters and device errors only (the record count stays until
+  // the donor phase: a call that is refused before it leaves the last records)
+  TB_CUDA(cudaMemsetAsync(call_words_.p, 0, (kCallWords - 1) * sizeof(unsigned long long), stream_));
   // the side stream is idle unless the last call stopped early (its pinned
   // staging is reused below); then the previous call's donor marks go back
   // to rest on it, beside everything up to the donor phase

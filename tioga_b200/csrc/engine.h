@@ -655,9 +655,10 @@ class Engine {
   long long excl_gen_ = -1;
   int excl_rounds_ = 0;
   DBuf<unsigned> obb_done_;  // per block: CTAs of the current OBB pass that have arrived
-  // the call's counters, zeroed together at its start and read back together
-  // at its end: counters_ (16 words), err_ (this call's error bits, a scratch
-  // word), scount_ (candidate overflows, refinements), rcount_ (records), nact_ (live leaf groups)
+  // the call's counters, zeroed together at its start (the last at the donor
+  // phase's) and read back together at its end: counters_ (16 words), err_ (this
+  // call's error bits, a scratch word), scount_ (candidate overflows,
+  // refinements), nact_ (live leaf groups), rcount_ (records)
   static constexpr int kCallWords = 20;
   DBuf<unsigned long long> call_words_;
   DView<unsigned long long> counters_;

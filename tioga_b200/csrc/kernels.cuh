@@ -205,7 +205,7 @@ __global__ void k_classify_tiles(const double* x, const BlockInfo* bi, int nb, c
                                  const float4* tbox, const int* node_order, const int* slot, int K,
                                  const HoleMapDev* hm, int* iblank, unsigned char* m0, int* m1, int* mlist,
                                  int* dcnt, unsigned long long* counters);
-__global__ void k_front_init(int* dcnt);
+__global__ void k_front_init(int* dcnt, int* rcount);
 __global__ void k_dilate_front(int iter, const int* csr_off, const int* csr_cell, const int* conn8,
                                const unsigned char* cell_nv, const blk_t* cell_blk, const BlockInfo* bi,
                                const unsigned char* m0, int* m1, int* mlist, int* dcnt);

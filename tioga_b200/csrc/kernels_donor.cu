@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(256) k_classify_tiles(
 }
 
 // frontier bounds of the nfringe layers: seg[0..1] and seg[2..3] alternate
-__global__ void k_front_init(int* __restrict__ dcnt) {
+__global__ void k_front_init(int* __restrict__ dcnt, int* __restrict__ rcount) {
+  *rcount = 0;  // (k_select counts the records)
   dcnt[kHoles] = dcnt[kMarked];
   dcnt[kSeg] = 0;
   dcnt[kSeg + 1] = dcnt[kMarked];
