@@ -297,7 +297,8 @@ void tioga_b200_getcelliblank_(int *btag, int *iblank_cell);
  * [13] query points merged into a coincident one (uniqNodesTree). */
 void tioga_b200_stats_(long long out[16]);
 /* More counters of the last connectivity call: [0] cells of its hole maps,
- * [1] cells whose boxes it made (the split form makes those near a receptor). */
+ * [1] cells whose boxes it made (those near a receptor where leaf groups were
+ * culled, else all). */
 void tioga_b200_stats2_(long long out[8]);
 /* Run on the caller's CUDA stream (a cudaStream_t; NULL restores the
  * library's own stream), e.g. to time the calls with the caller's events. */

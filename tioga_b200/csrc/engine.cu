@@ -1123,7 +1123,8 @@ int Engine::preprocess_resolutions(bool planned) {
                                                        d_bi_.p, ntot_, planned ? mand_.p : nullptr, node_res_.p);
   TB_LAUNCHED("k_node_res");
   if (planned) {
-    k_pre_finish<<<grid_for(std::max(ctot_, ntot_), kT), kT, 0, stream_>>>(excl_.p, ctot_, cell_res_.p, iblank_.p, ntot_);
+    k_pre_finish<<<grid_for(std::max(ctot_, ntot_), kT), kT, 0, stream_>>>(excl_.p, ctot_, cell_res_.p, iblank_.p,
+                                                                           ntot_);
     TB_LAUNCHED("k_pre_finish");
     return 0;
   }
@@ -1236,8 +1237,8 @@ int Engine::run_pairs_and_refit() {
   const unsigned ntiles = (unsigned)h_tile_base_.back();
   if (ntiles > 0 && !tiles_ready_) {  // (else made during the chunked upload)
     k_node_tiles<<<ntiles, 256, 0, stream_>>>(x_.p, d_bi_.p, nb, tile_base_.p, tbox_.p, node_order_.p,
-                                              boxes && !cull && !fp64 ? xf_.p : nullptr, nullptr, part_box_.p, part_need_.p,
-                                              blk_bnd_.p);
+                                              boxes && !cull && !fp64 ? xf_.p : nullptr, nullptr, part_box_.p,
+                                              part_need_.p, blk_bnd_.p);
     TB_LAUNCHED("k_node_tiles");
   }
   if (fp64) TB_CUDA(cbox64_.ensure(6 * ctot_));
@@ -1329,10 +1330,9 @@ int Engine::run_pairs_and_refit() {
   }
   TB_CUDA(cudaEventRecord(hev_[0], stream_));  // the hole maps may start
   TB_CUDA(cudaEventRecord(cev_[2], stream_));
-  launch_cell_pairs(fp64 ? 0 : 1, tune_.cell_pass_per_sm, ccta.back(), smem, stream_, x_.p, conn8_.p, cell_nv_.p, d_bi_.p,
-                    leaves_.p, d_chunks_.p, d_chunk_cta_.p, (int)chunks.size(), lw, d_pfirst_.p, d_pairs_.p,
-                    cull ? grp_live_.p : nullptr, cbox_.p, cbox64_.p,
-                    lbox_.p, pair_ext_.p, pair_acc_.p);
+  launch_cell_pairs(fp64 ? 0 : 1, tune_.cell_pass_per_sm, ccta.back(), smem, stream_, x_.p, conn8_.p, cell_nv_.p,
+                    d_bi_.p, leaves_.p, d_chunks_.p, d_chunk_cta_.p, (int)chunks.size(), lw, d_pfirst_.p, d_pairs_.p,
+                    cull ? grp_live_.p : nullptr, cbox_.p, cbox64_.p, lbox_.p, pair_ext_.p, pair_acc_.p);
   TB_LAUNCHED("k_leaf_seeds");
   TB_LAUNCHED("k_cell_pass");
   TB_CUDA(cudaEventRecord(cev_[1], stream_));
@@ -1420,8 +1420,9 @@ int Engine::run_search() {
   TB_CUDA(cudaEventRecord(sev_[1], stream_));
   if (count > 0) {
     TB_CUDA(refine_.ensure(count));
-    launch_candidates(form, grid_for(count, 256, 148 * tune_.candidates_per_sm), stream_, x_.p, conn8_.p, cell_nv_.p, cell_res_.p, sorted_cell_.p,
-                      qnode_.p, cand_.p, (int)count, qkey_.p, qacc_.p, refine_.p, scount_.p + 1, counters_.p);
+    launch_candidates(form, grid_for(count, 256, 148 * tune_.candidates_per_sm), stream_, x_.p, conn8_.p, cell_nv_.p,
+                      cell_res_.p, sorted_cell_.p, qnode_.p, cand_.p, (int)count, qkey_.p, qacc_.p, refine_.p,
+                      scount_.p + 1, counters_.p);
     TB_LAUNCHED("k_candidates");
     TB_CUDA(cudaEventRecord(sev_[2], stream_));
     if (form == 1) {
@@ -1477,10 +1478,10 @@ int Engine::traverse_and_gather(const double* xq, const int* qn, const int* qd, 
     if (attempt > 0 || !qkey)  // (zero at the start of a connectivity call)
       TB_CUDA(cudaMemsetAsync(scount_.p, 0, sizeof(unsigned), stream_));
     const bool quads = traverse_quads(form, tune_.traverse_variant, nq);
-    launch_traverse(form, tune_.traverse_variant, grid_for(quads ? 4 * nq : nq, 64, (quads ? 16 : 4) * 148 * tune_.traverse_per_sm), stream_, xq,
-                    d_bi_.p, cbox_.p,
-                    form == 0 ? cbox64_.p : nullptr, tnode_.p, qn, qd, nq,
-                    slots_.p, ncand_q_.p, ovf_.p, (int)ovf_cap, scount_.p, err_.p, skip_uhex, q_rep, qkey, qacc);
+    const int ctas = grid_for(quads ? 4 * nq : nq, 64, (quads ? 16 : 4) * 148 * tune_.traverse_per_sm);
+    launch_traverse(form, tune_.traverse_variant, ctas, stream_, xq, d_bi_.p, cbox_.p,
+                    form == 0 ? cbox64_.p : nullptr, tnode_.p, qn, qd, nq, slots_.p, ncand_q_.p, ovf_.p, (int)ovf_cap,
+                    scount_.p, err_.p, skip_uhex, q_rep, qkey, qacc);
     TB_LAUNCHED("k_traverse");
     size_t tmp = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tmp, ncand_q_.p, cand_off_.p, (int)(nq + 1), stream_);
@@ -1586,12 +1587,8 @@ int Engine::run_gid_merge() {
   qoff[npairs_] = (int)n;
   // the donors' lists in the reference's order: position i holds query refq[i]
   const int np = npairs_;
-  std::vector<int> prank(np), seen(hb_.size(), 0);
-  for (int p = 0; p < np; p++) prank[p] = seen[h_pairs_[p].don]++;
   TB_CUDA(dd_pqoff_.ensure(np + 1));
-  TB_CUDA(dd_prank_.ensure(np));
   TB_CUDA(cudaMemcpyAsync(dd_pqoff_.p, qoff.data(), (np + 1) * sizeof(int), cudaMemcpyHostToDevice, stream_));
-  TB_CUDA(cudaMemcpyAsync(dd_prank_.p, prank.data(), np * sizeof(int), cudaMemcpyHostToDevice, stream_));
   TB_CUDA(dd_key_.ensure(n));
   TB_CUDA(dd_key2_.ensure(n));
   TB_CUDA(dd_perm_.ensure(n));
@@ -1603,8 +1600,8 @@ int Engine::run_gid_merge() {
   TB_CUDA(q_gpos_.ensure(n));
   TB_CUDA(q_xt_.ensure(n));
   TB_CUDA(q_rep_.ensure(n));
-  k_dedup_keys<<<grid_for(n, kT), kT, 0, stream_>>>(qnode_.p, qdon_.p, n, dd_pqoff_.p, np, dd_prank_.p, node_bin_.p,
-                                                    bits_for(ntot_), dd_key_.p, dd_perm_.p);
+  k_dedup_keys<<<grid_for(n, kT), kT, 0, stream_>>>(qnode_.p, n, dd_pqoff_.p, np, node_bin_.p, bits_for(ntot_),
+                                                    dd_key_.p, dd_perm_.p);
   TB_LAUNCHED("k_dedup_keys");
   size_t tmp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tmp, dd_key_.p, dd_key2_.p, dd_perm_.p, dd_refq_.p, (int)n, 0, 64, stream_);
@@ -1665,14 +1662,9 @@ int Engine::run_gid_merge() {
 int Engine::dedup_merge(const DedupQueries& Qd, const std::vector<int>& qoff) {
   const long long n = Qd.n;
   const int np = npairs_;
-  std::vector<int> prank(np);
   const int nb = (int)hb_.size();
   std::vector<long long> dcount(nb, 0);
-  std::vector<int> seen(nb, 0);
-  for (int p = 0; p < np; p++) {
-    prank[p] = seen[h_pairs_[p].don]++;
-    dcount[h_pairs_[p].don] += qoff[p + 1] - qoff[p];
-  }
+  for (int p = 0; p < np; p++) dcount[h_pairs_[p].don] += qoff[p + 1] - qoff[p];
   // the donors' lists, first to last
   std::vector<int2> lists;
   long long pos = 0;
@@ -1683,11 +1675,9 @@ int Engine::dedup_merge(const DedupQueries& Qd, const std::vector<int>& qoff) {
   const int nlists = (int)lists.size();
   const size_t nseg_cap = (size_t)(n / (kDedupLeaf + 1)) + nlists + 1;  // active subsets of a level
   TB_CUDA(dd_pqoff_.ensure(np + 1));
-  TB_CUDA(dd_prank_.ensure(np));
   TB_CUDA(dd_lists_.ensure(nlists));
   TB_CUDA(dd_list_seg_.ensure(nlists));
   TB_CUDA(cudaMemcpyAsync(dd_pqoff_.p, qoff.data(), (np + 1) * sizeof(int), cudaMemcpyHostToDevice, stream_));
-  TB_CUDA(cudaMemcpyAsync(dd_prank_.p, prank.data(), np * sizeof(int), cudaMemcpyHostToDevice, stream_));
   TB_CUDA(cudaMemcpyAsync(dd_lists_.p, lists.data(), nlists * sizeof(int2), cudaMemcpyHostToDevice, stream_));
   TB_CUDA(dd_key_.ensure(n));
   TB_CUDA(dd_key2_.ensure(n));
@@ -1715,14 +1705,14 @@ int Engine::dedup_merge(const DedupQueries& Qd, const std::vector<int>& qoff) {
   if (Qd.qpt_local) {
     const int point_bits = bits_for(Qd.npoints);
     key_bits += point_bits;
-    k_dedup_keys_pts<<<grid_for(n, kT), kT, 0, stream_>>>(Qd.qpt_local, Qd.qdon, n, dd_pqoff_.p, np, dd_prank_.p,
-                                                          point_bits, dd_key_.p, dd_perm_.p);
+    k_dedup_keys_pts<<<grid_for(n, kT), kT, 0, stream_>>>(Qd.qpt_local, n, dd_pqoff_.p, np, point_bits,
+                                                          dd_key_.p, dd_perm_.p);
     TB_LAUNCHED("k_dedup_keys_pts");
   } else {
     const int node_bits = bits_for(ntot_);
     key_bits += node_bits + 10;
-    k_dedup_keys<<<grid_for(n, kT), kT, 0, stream_>>>(Qd.qid, Qd.qdon, n, dd_pqoff_.p, np, dd_prank_.p,
-                                                      node_bin_.p, node_bits, dd_key_.p, dd_perm_.p);
+    k_dedup_keys<<<grid_for(n, kT), kT, 0, stream_>>>(Qd.qid, n, dd_pqoff_.p, np, node_bin_.p, node_bits,
+                                                      dd_key_.p, dd_perm_.p);
     TB_LAUNCHED("k_dedup_keys");
   }
   size_t tmp = 0;

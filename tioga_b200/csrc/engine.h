@@ -46,8 +46,8 @@ inline bool traverse_quads(int form, int variant, long long nq) {
 constexpr int kSlots = 8;       // inline search candidates per query
 constexpr int kMaxBlocks = 100; // MAXBLOCKS, src/globals.h:29
 constexpr int kMaxSysBlocks = 16;      // blocks of one overset system (donor lists per node)
-constexpr int kMaxEngineBlocks = 8192;
-constexpr size_t kHoleMapCap = 197ull * 197ull * 197ull;  // bytes of one hole map at most // blocks of all systems of one engine (16-bit block ids)
+constexpr int kMaxEngineBlocks = 8192;  // blocks of all systems of one engine (16-bit block ids)
+constexpr size_t kHoleMapCap = 197ull * 197ull * 197ull;  // bytes of one hole map at most (6-neighbour mode)
 
 // Page-locked host memory that grows: copies to and from it do not hold the
 // host (a 4-byte read-back into pageable memory costs 14 us, into this 5).
@@ -264,7 +264,7 @@ struct Timing {
         total = 0, upload = 0, download = 0;
   float traverse = 0, candidates = 0, refine = 0;  // stages of the search
   float cell_pass = 0;                              // the cell pass kernel(s) alone
-  float cell_boxes = 0;                             // split form: its box kernel alone
+  float cell_boxes = 0;                             // its box kernel alone
 };
 
 class Engine {
@@ -506,7 +506,7 @@ class Engine {
   bool boxes_ready_ = false;              // this call's cell boxes were made during the upload
   bool tiles_ready_ = false;              // and its node tiles' boxes
   cudaEvent_t sev_[4];
-  cudaEvent_t cev_[3];  // around the cell pass (split form: and between its two kernels)
+  cudaEvent_t cev_[3];  // around the cell pass, and between its boxes and its pairs
   cudaEvent_t pev_;     // the pairs' copy to the host has landed
   bool cell_timed_ = false;
 
@@ -522,7 +522,8 @@ class Engine {
   bool dedup_active_ = false;       // some block has nodes within the gate's distance
   bool gate_valid_ = false;         // the gate holds for the device coordinates (moved rigidly since)
   bool dedup_ran_ = false;          // this call merged coincident query points
-  DBuf<int> q_xt_, q_rep_, q_gpos_, dd_refq_, dd_perm_, dd_perm2_, dd_mtag_, dd_itag_, dd_seg_, dd_seg2_, dd_member_, dd_cnt_, dd_ireset_;
+  DBuf<int> q_xt_, q_rep_, q_gpos_, dd_refq_, dd_perm_, dd_perm2_, dd_mtag_, dd_itag_, dd_seg_, dd_seg2_;
+  DBuf<int> dd_member_, dd_cnt_, dd_ireset_;
   DBuf<double> dd_x_, dd_rtag_;
   DBuf<unsigned long long> dd_key_, dd_key2_;
   DBuf<DedupSeg> dd_S_, dd_T_;
@@ -531,14 +532,15 @@ class Engine {
   DBuf<int> cg_table_;              // preprocess gate: hash table of node ids, its flag
   DBuf<unsigned> cg_flag_;
   DBuf<int4> dd_leaves_;
-  DBuf<int> dd_pqoff_, dd_prank_, dd_list_seg_;
+  DBuf<int> dd_pqoff_, dd_list_seg_;
   // high-order path
   std::vector<HoBlockDesc> ho_;
   bool ihigh_ = false, ihigh_global_ = false, ho_done_ = false;
   bool ho_dof_on_device_ = false;  // ho_xdof_ holds the registered DOF coordinates
   DBuf<HoDev> ho_dev_;
   DBuf<double> ho_xdof_, ho_pts_, ho_qres_, ho_w_, ho_q_, ho_qtmp_, ho_qu_;
-  DBuf<int> ho_ctag_, ho_rcblk_, ho_qpt_, ho_qloc_, ho_qdon_, ho_qrec_, ho_qbest_, ho_npass_, ho_qcell_, ho_win_, ho_flag_, ho_off_;
+  DBuf<int> ho_ctag_, ho_rcblk_, ho_qpt_, ho_qloc_, ho_qdon_, ho_qrec_, ho_qbest_, ho_npass_, ho_qcell_, ho_win_;
+  DBuf<int> ho_flag_, ho_off_;
   DBuf<long long> ho_rcoff_d_, ho_ptoff_d_;
   DBuf<int4> ho_rec_;
   std::vector<long long> ho_rc_off_, ho_pt_off_;
@@ -585,8 +587,8 @@ class Engine {
   // tree
   DBuf<int> sorted_cell_;
   DBuf<float2> cbox_;      // split form: 3 per sorted cell (FP32 box rounded outward, 24 bytes)
-  DBuf<float4> lbox_;      // split form: 2 per leaf, in leaf order (its box, and its block in the 7th word)
-  DBuf<int> pair_ext_;     // split form: 6 per pair, the seeds of the extents' bounds (fkey order)
+  DBuf<float4> lbox_;      // 2 per leaf, in leaf order (its box, and its block in the 7th word)
+  DBuf<int> pair_ext_;     // 6 per pair, the seeds of the extents' bounds (fkey order)
   DBuf<float4> xf_;        // coordinates rounded to FP32, one per node (split-form cell boxes)
   // leaf groups (k_group_cull): node parts per group, this call's live ones
   DBuf<int2> grp_;

@@ -340,7 +340,8 @@ int Engine::connectivity_highorder() {
     ho_dof_on_device_ = true;
   }
   // receptor cells (getInternalNodes, highOrder.C:208-247)
-  DBuf<int>&flag = ho_flag_, &off = ho_off_;
+  DBuf<int>& flag = ho_flag_;
+  DBuf<int>& off = ho_off_;
   TB_CUDA(flag.ensure(ctot_ + 1));
   TB_CUDA(off.ensure(ctot_ + 1));
   k_ho_rcflag<<<grid_for(ctot_, kT), kT, 0, stream_>>>(iblank_cell_.p, inv_sorted_.p, ctot_, flag.p);
@@ -489,7 +490,8 @@ int Engine::connectivity_highorder() {
   if (nr > 0) {
     k_ho_records<<<grid_for(nq, 128), 128, 0, stream_>>>(flag.p, off.p, nq, ho_qcell_.p, ho_qdon_.p, ho_qrec_.p,
                                                          ho_qloc_.p, ho_qpt_.p, ho_pts_.p, ho_dev_.p, ho_xdof_.p,
-                                                         q_rep_.p, ho_npass_.p, ho_qu_.p, ho_wstride_, ho_rec_.p, ho_w_.p);
+                                                         q_rep_.p, ho_npass_.p, ho_qu_.p, ho_wstride_, ho_rec_.p,
+                                                         ho_w_.p);
     TB_LAUNCHED("k_ho_records");
   }
   ho_nrecs_ = nr;

@@ -191,8 +191,8 @@ __global__ void k_uhex_search(const double* x, const int* qnode, const int* qdon
 // ---- donors (kernels_donor.cu) ----
 __global__ void k_fill_slots(const int* qnode, const int* qdon, const int* qcell, long long nq, DonorSlots slots,
                              unsigned* err);
-__global__ void k_donor_rest(long long ntot, long long ctot, int K, unsigned char* m0, int* m1, int* cmark, int* reset_t,
-                             int* slot, int* iblank_cell, int* dcnt);
+__global__ void k_donor_rest(long long ntot, long long ctot, int K, unsigned char* m0, int* m1, int* cmark,
+                             int* reset_t, int* slot, int* iblank_cell, int* dcnt);
 __global__ void k_write_iblanks(const int* iblank, const blk_t* node_blk, long long ntot, int* const* dst);
 __global__ void k_donor_reset(const int* mlist, const int* dcnt, const int* it_rec, const unsigned char* it_cancel,
                               int prev_R, const int* csr_off, const int* csr_cell, int* iblank, unsigned char* m0,
@@ -224,17 +224,16 @@ __global__ void k_interp(const double* x, const unsigned long long* rkey, const 
                          const int* reset_t, const int* orig_cell, int* it_node, double* it_w, int* it_rec,
                          int* it_don, unsigned char* it_nv, unsigned char* it_cancel, double* rres, int* interp2rec,
                          unsigned* err);
-__global__ void k_coin_hash(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot, short* node_bin,
-                            int* table, unsigned mask, unsigned* flag);
+__global__ void k_coin_hash(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot,
+                            short* node_bin, int* table, unsigned mask, unsigned* flag);
 __global__ void k_coin_file(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot, int* table,
                             unsigned mask, unsigned* flag);
 __global__ void k_coin_compare(const double* x, const blk_t* node_blk, const BlockInfo* bi, long long ntot,
                                const int* table, unsigned mask, unsigned* flag);
-__global__ void k_dedup_keys(const int* qnode, const int* qdon, long long nq, const int* pair_qoff, int npairs,
-                             const int* pair_rank, const short* node_bin, int node_bits, unsigned long long* key,
-                             int* val);
-__global__ void k_dedup_keys_pts(const int* qpt_local, const int* qdon, long long nq, const int* pair_qoff,
-                                 int npairs, const int* pair_rank, int point_bits, unsigned long long* key, int* val);
+__global__ void k_dedup_keys(const int* qnode, long long nq, const int* pair_qoff, int npairs, const short* node_bin,
+                             int node_bits, unsigned long long* key, int* val);
+__global__ void k_dedup_keys_pts(const int* qpt_local, long long nq, const int* pair_qoff, int npairs, int point_bits,
+                                 unsigned long long* key, int* val);
 __global__ void k_dedup_start(const int2* lists, int nlists, DedupSeg* S, int* seg_of_list, int4* leaves, int* cnt);
 __global__ void k_dedup_gather(const int* refq, long long n, const int* qnode, const double* qres, const double* x,
                                const blk_t* node_blk, const int* qrec, const BlockInfo* bi, const int2* lists,

@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(256) k_wall_setup(const double* __restrict__ x
 
 // wall-touching cells mark their index box with 2 (MeshBlock.C:666-772):
 // one thread per cell of the wall-cell list (cells of wall-bearing blocks
-// with a wall node).  Maps past the slab are left alone (the host rejects
-// such a map before it is used).
+// with a wall node).  Maps past the slab would be left alone; k_wall_setup
+// clamps their sizes to it and reports kErrBadIndex.
 __global__ void k_holemap_mark(const double* __restrict__ x, const int* __restrict__ conn8,
                                const unsigned char* __restrict__ cell_nv, const int* __restrict__ wall_cells,
                                int nwc, const blk_t* __restrict__ cell_blk, const BlockInfo* __restrict__ bi,
@@ -506,7 +506,7 @@ __device__ int obb_intersect(const double vA[3][3], const double xA[3], const do
 // order.  pfirst[b] = first pair whose donor is block b (pairs are sorted by
 // donor), pfirst[nb] = the pair count.  The pairs' extents start here too:
 // acc at BIG / -BIG as getReducedOBB does (MeshBlock.C:790-794, ordered keys),
-// ext (the split form's bounds) open, and every block's node bounds
+// ext (the leaf seeds' bounds) open, and every block's node bounds
 // (k_node_tiles) open.
 constexpr int kPairThreads = 1024;
 __global__ void __launch_bounds__(kPairThreads) k_pairs(const BlockInfo* __restrict__ bi, int nb,
@@ -595,8 +595,8 @@ __global__ void k_pair_finish(const BlockInfo* __restrict__ bi, PairInfo* __rest
 // block, so what they are rounded to goes with the block's size and not with
 // its distance from the origin: with cells of 1/128 at 2^20 every walk visited
 // thousands of cells (22 k queries 10.85 ms, 0.07 ms with it and at the
-// origin; with FP64 boxes in the tree 0.22 ms in both places).  A box holds a point after the subtraction if it did before, as
-// rounding keeps the order.
+// origin; with FP64 boxes in the tree 0.22 ms in both places).  A box holds a
+// point after the subtraction if it did before, as rounding keeps the order.
 __device__ __forceinline__ double tree_origin(const BlockInfo& B, int k) {
   return isfinite(B.obb.xc[k]) ? B.obb.xc[k] : 0.0;
 }
@@ -920,7 +920,7 @@ __device__ __forceinline__ void cell_box_load(const float2* __restrict__ cbox, l
 // nleaf leaves listed there (those whose coordinates have been uploaded), with
 // act the *nact leaf groups listed there (k_group_cull's).  FORM 0 takes the
 // FP64 coordinates and keeps the exact FP64 boxes of the cells (cbox64); the
-// leaves' are rounded outward.  (One kernel over boxes and pairs, with the
+// leaves' are rounded outward, in the tree relative to their block.  (One kernel over boxes and pairs, with the
 // registers of both, took 176 us of the FP64 form's call on 1.8 M nodes; the
 // three take 167 us and one code path.)
 template <int MINB, int FORM>
@@ -1073,7 +1073,8 @@ __global__ void __launch_bounds__(256, MINB) k_cell_pairs(
     const BlockInfo* __restrict__ bi, const int4* __restrict__ leaves, const int4* __restrict__ chunks,
     const int* __restrict__ chunk_cta, int nchunks, int lw, const int* __restrict__ pfirst,
     const PairInfo* __restrict__ pairs, const unsigned char* __restrict__ live, const float2* __restrict__ cbox,
-    const double* __restrict__ cbox64,    const float4* __restrict__ lbox, const int* __restrict__ ext, unsigned long long* __restrict__ acc) {
+    const double* __restrict__ cbox64, const float4* __restrict__ lbox, const int* __restrict__ ext,
+    unsigned long long* __restrict__ acc) {
   extern __shared__ unsigned long long s_dyn[];
   int cta, ncta;
   const int kc = chunk_of_cta(chunk_cta, nchunks);
@@ -1222,8 +1223,8 @@ void launch_cell_boxes(int form, int minb, int grid, cudaStream_t st, const doub
 void launch_cell_pairs(int form, int minb, int grid, size_t smem, cudaStream_t st, const double* x, const int* conn8,
                        const unsigned char* cell_nv, const BlockInfo* bi, const int4* leaves, const int4* chunks,
                        const int* chunk_cta, int nchunks, int lw, const int* pfirst, const PairInfo* pairs,
-                       const unsigned char* live, const float2* cbox, const double* cbox64, const float4* lbox, int* ext,
-                       unsigned long long* acc) {
+                       const unsigned char* live, const float2* cbox, const double* cbox64, const float4* lbox,
+                       int* ext, unsigned long long* acc) {
   set_smem(k_leaf_seeds, smem);
   k_leaf_seeds<<<grid, 256, smem, st>>>(bi, chunks, chunk_cta, nchunks, lw, pfirst, pairs, live, lbox, ext);
 #define TB_CPP(MB, F)                                                                                     \
@@ -2420,21 +2421,22 @@ void launch_traverse(int form, int variant, int blocks, cudaStream_t st, const d
                      const int* qnode, const int* qdon, long long nq, int* slots, int* ncand_q, int3* ovf,
                      int ovf_cap, unsigned* novf, unsigned* err, int skip_uhex, const int* q_rep,
                      unsigned long long* qkey, unsigned* qacc) {
+  const bool quads = traverse_quads(form, variant, nq);
   if (form == 1 && variant == 1)
-    k_traverse_ww<<<blocks, kWalkThreads, 0, st>>>(x, bi, cbox, tnode, qnode, qdon, nq, slots, ncand_q, ovf, ovf_cap, novf,
-                                          err, skip_uhex, q_rep, qkey, qacc);
-  else if (traverse_quads(form, variant, nq) && form == 0)
+    k_traverse_ww<<<blocks, kWalkThreads, 0, st>>>(x, bi, cbox, tnode, qnode, qdon, nq, slots, ncand_q,
+                                                   ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
+  else if (quads && form == 0)
     k_traverse_quad<0><<<blocks, kWalkThreads, 0, st>>>(x, bi, cbox, cbox64, tnode, qnode, qdon, nq, slots, ncand_q,
-                                          ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
-  else if (traverse_quads(form, variant, nq))
+                                                        ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
+  else if (quads)
     k_traverse_quad<1><<<blocks, kWalkThreads, 0, st>>>(x, bi, cbox, cbox64, tnode, qnode, qdon, nq, slots, ncand_q,
-                                          ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
+                                                        ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
   else if (form == 0)
     k_traverse<0><<<blocks, kWalkThreads, 0, st>>>(x, bi, cbox, cbox64, tnode, qnode, qdon, nq, slots, ncand_q,
-                                          ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
+                                                   ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
   else
     k_traverse<1><<<blocks, kWalkThreads, 0, st>>>(x, bi, cbox, cbox64, tnode, qnode, qdon, nq, slots, ncand_q,
-                                          ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
+                                                   ovf, ovf_cap, novf, err, skip_uhex, q_rep, qkey, qacc);
 }
 
 void launch_candidates(int form, int blocks, cudaStream_t st, const double* x, const int* conn8,

@@ -73,7 +73,7 @@ constexpr int kCoinBits = 17;      // delta is a quarter of a cell of 2^17 per a
 constexpr int kCoinCoarse = 8;     // width of a filing cell in those cells
 constexpr int kCoinWalk = 128;     // a longer walk counts as crowded
 constexpr double kCoinFine = 2.01; // width of a crowded gate's cells in delta
-constexpr int kCoinProbes = 4096;  // there a longer walk counts as close nodes (the merge then runs, to the same result)
+constexpr int kCoinProbes = 4096;  // there a longer walk counts as close nodes (the merge then runs)
 constexpr unsigned kCoinClose = 1u, kCoinCrowded = 2u;  // the gate's flag
 
 // delta of a block, and a cell's place in the table
@@ -178,7 +178,8 @@ __global__ void k_coin_compare(const double* __restrict__ x, const blk_t* __rest
     const int b = node_blk[g];
     const double p[3] = {x[3 * g], x[3 * g + 1], x[3 * g + 2]};
     const double delta = coin_delta(bi[b]), inv = 1.0 / (kCoinFine * delta);
-    constexpr double reach = 0.498;  // delta in cells (1 / 2.01), with room for the rounding; a node's box touches two at most
+    // delta in cells (1 / 2.01), with room for the rounding; a node's box touches two an axis at most
+    constexpr double reach = 0.498;
     int c0[3], c1[3];
     for (int k = 0; k < 3; k++) {
       const double t = (p[k] - (double)bi[b].bb_lo[k]) * inv + 0.37;
@@ -205,11 +206,9 @@ __global__ void k_coin_compare(const double* __restrict__ x, const blk_t* __rest
 // donor block, so a donor's pairs are consecutive and in list order); sorting
 // the queries by it gives every donor's list in the reference's order (gpos =
 // position in that sorted order)
-__global__ void k_dedup_keys(const int* __restrict__ qnode, const int* __restrict__ qdon, long long nq,
-                             const int* __restrict__ pair_qoff, int npairs, const int* __restrict__ pair_rank,
-                             const short* __restrict__ node_bin, int node_bits,
-                             unsigned long long* __restrict__ key,
-                             int* __restrict__ val) {
+__global__ void k_dedup_keys(const int* __restrict__ qnode, long long nq, const int* __restrict__ pair_qoff,
+                             int npairs, const short* __restrict__ node_bin, int node_bits,
+                             unsigned long long* __restrict__ key, int* __restrict__ val) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq;
        q += (long long)gridDim.x * blockDim.x) {
     int lo = 0, hi = npairs - 1;  // the last pair whose first query is <= q
@@ -227,9 +226,9 @@ __global__ void k_dedup_keys(const int* __restrict__ qnode, const int* __restric
 
 // the same for the high-order path's receptor points: within a pair the
 // donor list holds them in point order (getExtraQueryPoints, highOrder.C:272-319)
-__global__ void k_dedup_keys_pts(const int* __restrict__ qpt_local, const int* __restrict__ qdon, long long nq,
-                                 const int* __restrict__ pair_qoff, int npairs, const int* __restrict__ pair_rank, int point_bits,
-                                 unsigned long long* __restrict__ key, int* __restrict__ val) {
+__global__ void k_dedup_keys_pts(const int* __restrict__ qpt_local, long long nq, const int* __restrict__ pair_qoff,
+                                 int npairs, int point_bits, unsigned long long* __restrict__ key,
+                                 int* __restrict__ val) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq;
        q += (long long)gridDim.x * blockDim.x) {
     int lo = 0, hi = npairs - 1;

@@ -383,7 +383,8 @@ __device__ void obb_finish(const double r[12], int pass, const double* __restric
 // twelve: the finish, a launch of its own with 148 x 12 dependent loads on
 // one thread, took 52-59 us a pass and the partial 8-13 us.
 __global__ void __launch_bounds__(256) k_obb_pass(const double* __restrict__ x, BlockInfo* __restrict__ bi_all,
-                                                  int pass, double* __restrict__ part_all, unsigned* __restrict__ done) {
+                                                  int pass, double* __restrict__ part_all,
+                                                  unsigned* __restrict__ done) {
   __shared__ double sh[256 * 12];
   __shared__ bool s_last;
   BlockInfo* bi = bi_all + blockIdx.y;
