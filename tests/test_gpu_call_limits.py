@@ -340,3 +340,45 @@ def test_update_after_a_refused_connectivity_call(side, oracle_lib):
         for b, a in zip(system.blocks, q):
             assert np.array_equal(a.cpu().numpy().view(np.int64), ref["q"][b.tag].view(np.int64))
     t.delete()
+
+
+@pytest.mark.parametrize("nvar", [40, 360])
+def test_columns_of_page_locked_fields(nvar, oracle_lib):
+    """Column-layout updates on either side of the line from which page-locked
+    fields go up whole, page-locked throughout, in part and not at all: the
+    same bits, and on the small side the oracle's."""
+    import torch
+    system = cases.config1(3, nbg=45, nshell=2, nr=7, nt=11, nphi=21, split_layers=2)
+    n = sum(b.nnodes for b in system.blocks)
+    assert n * 40 < 1 << 25 <= n * 360
+    rng = np.random.default_rng(nvar)
+    q0 = [rng.standard_normal(b.nnodes * nvar) for b in system.blocks]
+    t = _connected(system)
+    got = []
+    for pinned in ((False, False, False), (True, True, True), (True, False, True)):
+        q = [torch.from_numpy(a.copy()) for a in q0]
+        q = [a.pin_memory() if p else a for a, p in zip(q, pinned)]
+        for b, a in zip(system.blocks, q):
+            t.lib.tioga_registersolution_(C.byref(C.c_int(b.tag)), C.c_void_p(a.data_ptr()))
+        for _ in range(2):
+            t.dataupdate_mb(nvar, "column")
+            assert t.lib.tioga_b200_last_error() == 0
+        got.append([a.numpy() for a in q])
+    t.delete()
+    for g in got[1:]:
+        for a, b in zip(got[0], g):
+            assert np.array_equal(a.view(np.int64), b.view(np.int64))
+    if nvar == 40:
+        ref = TiogaLibrary(oracle_lib)
+        ref.init()
+        ref.register_system(system)
+        ref.preprocess_grids()
+        ref.performconnectivity()
+        q = [a.copy() for a in q0]
+        for b, a in zip(system.blocks, q):
+            ref.registersolution(b.tag, a)
+        for _ in range(2):
+            ref.dataupdate_mb(nvar, "column")
+        ref.delete()
+        for a, b in zip(got[1], q):
+            assert np.array_equal(a.view(np.int64), b.view(np.int64))

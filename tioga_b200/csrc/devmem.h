@@ -28,6 +28,19 @@ inline bool kernel_reaches(const void* p, int dev, size_t align) {
   return kernel_reaches(a, dev, p, align);
 }
 
+// Whether a host array is page-locked (from its first byte to its last).
+inline bool page_locked(const void* p, size_t bytes) {
+  for (const char* c : {static_cast<const char*>(p), static_cast<const char*>(p) + (bytes ? bytes - 1 : 0)}) {
+    cudaPointerAttributes a = {};
+    if (!p || cudaPointerGetAttributes(&a, c) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type != cudaMemoryTypeHost) return false;
+  }
+  return true;
+}
+
 // Device bytes of the engine whose calls this thread is running (the
 // serving form's admission accounting); null: not counted.
 extern thread_local long long* g_dbuf_account;

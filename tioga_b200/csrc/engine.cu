@@ -2571,9 +2571,27 @@ int Engine::dataupdate(int nvar, int interptype) {
   // and go up, a slot on its way while the next is packed, and the receptors'
   // values come back the same way.  Uploading every field from the caller's
   // pageable arrays took 6.8 of 12 ms on a system of 1.8 M nodes.
+  // Many large page-locked columns go up whole.
   TB_TRY(update_lists());
-  const int U = up_nodes_;
-  TB_CUDA(q_.ensure((size_t)U * nvar));
+  bool whole = interptype != 0 && columns_go_whole(ntot_, nvar);
+  for (size_t b = 0; b < hb_.size() && whole; b++)
+    whole = page_locked(hb_[b].hq, (size_t)hb_[b].nnodes * nvar * sizeof(double));
+  if (whole && q_.ensure((size_t)ntot_ * nvar) != cudaSuccess) {  // no room: packed all the same
+    cudaGetLastError();
+    whole = false;
+  }
+  const int U = whole ? 0 : up_nodes_;
+  if (whole) {
+    std::vector<double*> qptr(hb_.size());
+    for (size_t b = 0; b < hb_.size(); b++) {
+      qptr[b] = q_.p + (size_t)bi_[b].node_off * nvar;
+      TB_CUDA(cudaMemcpyAsync(qptr[b], hb_[b].hq, (size_t)hb_[b].nnodes * nvar * sizeof(double),
+                              cudaMemcpyHostToDevice, stream_));
+    }
+    TB_TRY(upload_qptr(qptr));
+  } else {
+    TB_CUDA(q_.ensure((size_t)U * nvar));
+  }
   const size_t row = nvar * sizeof(double);
   const int per = std::max(1, std::min((int)((1 << 20) / row), std::max(U, (int)nrec_)));  // rows of a slot
   TB_CUDA(h_up_slots_.ensure(2 * per * row));
@@ -2591,16 +2609,17 @@ int Engine::dataupdate(int nvar, int interptype) {
       int e = u;
       while (e < u1 && list[e] < end) e++;
       const double* q = hb_[blk].hq;
-      if (interptype == 0) {
+      if (interptype == 0 && nvar > 1) {
         for (int i = u; i < e; i++) {
           if (i + 24 < e) __builtin_prefetch(q + (size_t)(list[i + 24] - off) * nvar);
           std::memcpy(stage + (size_t)i * nvar, q + (size_t)(list[i] - off) * nvar, row);
         }
-      } else {
-        for (int k = 0; k < nvar; k++) {
-          const double* qk = q + (size_t)k * hb_[blk].nnodes;
-          for (int i = u; i < e; i++) stage[(size_t)i * nvar + k] = qk[list[i] - off];
-        }
+      } else {  // (32 nodes at a time, so that their rows stay in the first cache)
+        for (int i0 = u; i0 < e; i0 += 32)
+          for (int k = 0; k < nvar; k++) {
+            const double* qk = q + (size_t)k * hb_[blk].nnodes;
+            for (int i = i0; i < std::min(e, i0 + 32); i++) stage[(size_t)i * nvar + k] = qk[list[i] - off];
+          }
       }
       u = e;
     }
@@ -2609,8 +2628,9 @@ int Engine::dataupdate(int nvar, int interptype) {
     TB_CUDA(cudaEventRecord(up_slot_ev_[part & 1], stream_));
   }
   k_interp_gather<<<grid_for(nval, kT), kT, 0, stream_>>>(it_node_.p, it_w_.p, it_don_.p, it_nv_.p, it_cancel_.p,
-                                                          rcount_.p, d_bi_.p, nullptr, up_need_.p, up_off_.p, q_.p,
-                                                          nvar, interptype, qvals_.p);
+                                                          rcount_.p, d_bi_.p, whole ? d_qptr_.p : nullptr,
+                                                          whole ? nullptr : up_need_.p, up_off_.p, q_.p, nvar,
+                                                          interptype, qvals_.p);
   TB_LAUNCHED("k_interp_gather");
   // back, and into the caller's arrays (updateSolnData, dataUpdate.C:105-119)
   auto fetch = [&](long long r0, int slot) -> cudaError_t {

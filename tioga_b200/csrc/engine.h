@@ -43,6 +43,15 @@ constexpr long long kQuadQueries = 1 << 20;
 inline bool traverse_quads(int form, int variant, long long nq) {
   return !(form == 1 && variant == 1) && nq < kQuadQueries;
 }
+// A column-layout update of page-locked host fields takes them up whole where
+// the columns are past the host's caches and more of them are read at once than
+// its prefetchers follow, else only the donors' values, packed (any other
+// layout or memory too).  Whole and packed, in ms: 1.8 M nodes, 5 fields 2.0 and
+// 2.5, 6 fields 2.3 and 3.6, 20 fields 8.6 and 14.3; 1.2 M nodes, 6 fields 2.2
+// and 1.4; 340 k nodes, 20 fields 1.6 and 0.8; 0.7 M nodes, 50 fields 7.5 and 11.
+inline bool columns_go_whole(long long nodes, int nvar) {
+  return nvar >= 6 && (nodes >= 3 << 19 || nodes * nvar >= 1 << 25);
+}
 constexpr int kSlots = 8;       // inline search candidates per query
 constexpr int kMaxBlocks = 100; // MAXBLOCKS, src/globals.h:29
 constexpr int kMaxSysBlocks = 16;      // blocks of one overset system (donor lists per node)
