@@ -32,3 +32,10 @@ def test_kernels_work_on_arrays_of_their_own_device_only(tmp_path):
 def test_donor_slots_refuse_indices_outside_their_arrays(tmp_path):
     """Both kernels that fill the donor slots take their places from here."""
     _run(tmp_path, "donor_slots_check.cu", os.environ.get("NVCC", "nvcc"))
+
+
+def test_one_page_locked_allocation_per_instance(tmp_path):
+    """Each such allocation takes milliseconds: the small buffers and the data
+    update's slots share one, and outgrow it safely."""
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    _run(tmp_path, "pinned_check.cc", "g++", "-I", os.path.join(cuda, "include"))

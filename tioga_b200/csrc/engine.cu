@@ -74,6 +74,7 @@ Engine::~Engine() {
   for (auto& e : up_slot_ev_) cudaEventDestroy(e);
   h_tab_.release();
   h_rb_.release();
+  h_pin_.release();
   // (the device buffers, then their stream, go with the members; nothing uses
   // them any more)
   if (dev_pool_) dev_pool_->users.clear();
@@ -302,7 +303,7 @@ int Engine::upload_topology() {
   scount_.p = err_.p + 2;
   nact_.p = reinterpret_cast<unsigned*>(call_words_.p + 18);
   rcount_.p = reinterpret_cast<int*>(call_words_.p + 19);
-  TB_CUDA(h_rb_.ensure(1024));
+  TB_CUDA(h_rb_.ensure(1024, h_pin_));
   TB_CUDA(cudaMemsetAsync(wallf_.p, 0, ntot_, stream_));
   TB_CUDA(cudaMemsetAsync(obcf_.p, 0, ntot_, stream_));
   TB_CUDA(cudaMemsetAsync(call_words_.p, 0, kCallWords * sizeof(unsigned long long), stream_));
@@ -981,7 +982,7 @@ int Engine::preprocess() {
   // distance), so the gate of the last preprocess still holds after them
   const bool gate = !gate_valid_;
   const size_t bi_bytes = bi_.size() * sizeof(BlockInfo);
-  TB_CUDA(h_rb_.ensure(bi_bytes + 64));
+  TB_CUDA(h_rb_.ensure(bi_bytes + 64, h_pin_));
   TB_CUDA(vol_big_.ensure(1));
   if (gate) {
     TB_TRY(dedup_gate());
@@ -1217,7 +1218,7 @@ int Engine::run_pairs_and_refit() {
   TB_CUDA(pair_acc_.ensure(6 * (size_t)npcand_));
   TB_CUDA(pair_ext_.ensure(6 * (size_t)npcand_));
   const size_t o_first = 64, o_pairs = o_first + ((nb + 1) * sizeof(int) + 63) / 64 * 64;
-  TB_CUDA(h_rb_.ensure(o_pairs + npcand_ * sizeof(PairInfo)));
+  TB_CUDA(h_rb_.ensure(o_pairs + npcand_ * sizeof(PairInfo), h_pin_));
   k_pairs<<<1, 1024, 0, stream_>>>(d_bi_.p, nb, d_pcand_.p, npcand_, d_pairs_.p, d_npairs_.p, d_pfirst_.p,
                                    pair_acc_.p, pair_ext_.p, blk_bnd_.p);
   TB_LAUNCHED("k_pairs");
@@ -1310,7 +1311,7 @@ int Engine::run_pairs_and_refit() {
   // call, after this call's final synchronisation)
   const size_t b_t0 = (h_pair_t0_.size() * sizeof(long long) + 15) / 16 * 16, b_ch = chunks.size() * sizeof(int4),
                b_cta = ccta.size() * sizeof(int);
-  TB_CUDA(h_tab_.ensure(b_t0 + b_ch + b_cta));
+  TB_CUDA(h_tab_.ensure(b_t0 + b_ch + b_cta, h_pin_));
   TB_CUDA(d_tab_.ensure(b_t0 + b_ch + b_cta));
   memcpy(h_tab_.p, h_pair_t0_.data(), h_pair_t0_.size() * sizeof(long long));
   memcpy(h_tab_.p + b_t0, chunks.data(), b_ch);
@@ -2593,10 +2594,13 @@ int Engine::dataupdate(int nvar, int interptype) {
     TB_CUDA(q_.ensure((size_t)U * nvar));
   }
   const size_t row = nvar * sizeof(double);
-  const int per = std::max(1, std::min((int)((1 << 20) / row), std::max(U, (int)nrec_)));  // rows of a slot
-  TB_CUDA(h_up_slots_.ensure(2 * per * row));
-  double* const slots[2] = {reinterpret_cast<double*>(h_up_slots_.p),
-                            reinterpret_cast<double*>(h_up_slots_.p + per * row)};
+  const int per = std::max(1, std::min((int)(PinArena::kSlots / 2 / row), std::max(U, (int)nrec_)));  // rows of a slot
+  char* base = 2 * per * row <= PinArena::kSlots ? h_pin_.slots() : nullptr;
+  if (!base) {
+    TB_CUDA(h_up_slots_.ensure(2 * per * row, h_pin_));
+    base = h_up_slots_.p;
+  }
+  double* const slots[2] = {reinterpret_cast<double*>(base), reinterpret_cast<double*>(base + per * row)};
   const int* list = h_up_list_.data();
   size_t blk = 0;  // block of the current node (the list ascends)
   for (int u0 = 0, part = 0; u0 < U; u0 += per, part++) {

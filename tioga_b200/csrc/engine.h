@@ -58,26 +58,6 @@ constexpr int kMaxSysBlocks = 16;      // blocks of one overset system (donor li
 constexpr int kMaxEngineBlocks = 8192;  // blocks of all systems of one engine (16-bit block ids)
 constexpr size_t kHoleMapCap = 197ull * 197ull * 197ull;  // bytes of one hole map at most (6-neighbour mode)
 
-// Page-locked host memory that grows: copies to and from it do not hold the
-// host (a 4-byte read-back into pageable memory costs 14 us, into this 5).
-struct PinBuf {
-  char* p = nullptr;
-  size_t n = 0;
-  cudaError_t ensure(size_t bytes) {
-    if (bytes <= n) return cudaSuccess;
-    release();
-    const size_t c = bytes + bytes / 2 + 4096;
-    const cudaError_t e = cudaMallocHost((void**)&p, c);
-    if (e == cudaSuccess) n = c;
-    else p = nullptr;
-    return e;
-  }
-  void release() {
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    n = 0;
-  }
-};
 // a typed part of a DBuf
 template <class T>
 struct DView {
@@ -570,6 +550,7 @@ class Engine {
   // p, [pair_t0[p], pair_t0[p + 1]); cell pass: (first leaf, end leaf, first
   // pair, pairs) per chunk, and each chunk's first CTA
   DBuf<char> d_tab_;
+  PinArena h_pin_;
   PinBuf h_tab_;
   DView<long long> d_pair_t0_;
   DView<int4> d_chunks_;
@@ -646,8 +627,8 @@ class Engine {
   DBuf<unsigned> up_need_;            // a bit per node that a live record reads
   DBuf<int> up_cnt_, up_off_, up_list_, up_rec_;
   std::vector<int> h_up_list_, h_up_rec_;  // those nodes, the receptors (-1: cancelled)
-  // values pass through two pinned slots of up to 1 MB in turn (pinning memory
-  // for all of them cost a new mesh's first update 7 ms)
+  // values pass through two pinned slots in turn (pinning memory for all of
+  // them cost a new mesh's first update 7 ms), the arena's unless a row is larger
   PinBuf h_up_slots_;
   cudaEvent_t up_slot_ev_[2];         // the slot's copy is done
   int up_nodes_ = 0;
