@@ -146,7 +146,7 @@ cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 }
 
 int main() {
-  const size_t big = 64 << 20;
+  const size_t big = 1 << 20;
   cudaStream_t main_st, side;
   cudaStreamCreateWithFlags(&main_st, 0);
   cudaStreamCreateWithFlags(&side, 0);
@@ -188,6 +188,11 @@ int main() {
     a.release();
     S(main_st)->capturing = false;
     pool->users.clear();  // as at the engine's end
+    // large buffers do not come from the pool
+    tb::DBuf<char> large, below;
+    large.ensure(tb::DevPool::kDirect);
+    below.ensure(tb::DevPool::kDirect - 1);
+    expect(!large.dev && below.dev, "which buffers come from the pool");
   }
   pool.reset();
   expect(pools == 0, "the pool outlives its last buffer");

@@ -56,11 +56,17 @@ extern thread_local cudaMemPool_t g_dbuf_pool;
 // the C API drives.  A new mesh needs about 200 buffers, which cost 90 us each
 // with cudaMalloc and 80 us with cudaFree; the pool maps device memory in
 // larger pieces (a new mesh of 450 k nodes from registration to its first data
-// update and the end of the instance, medians of 24: 51 ms without a pool, 28
-// with it).  It is made for the first buffer, as a solver's set-up may end
-// before that, keeps up to kKeep bytes that no buffer uses, and goes back to the
-// device with the engine's last buffer.  (Keeping 2 or 8 GB leaves the first
-// call on 18.6 M nodes as it is: 8.8 to 9.9 ms, 13 without a pool.)
+// update and the end of the instance, medians of 30: 53 to 57 ms without a pool,
+// 25 to 28 with it).  It is made for the first buffer, as a solver's set-up may
+// end before that, keeps up to kKeep bytes that no buffer uses, and goes back to
+// the device with the engine's last buffer.
+//
+// Buffers of kDirect and more come from the device directly: mapping them is
+// what they cost, and a pool that gives back what it does not use maps some of
+// it again (18.6 M nodes, first preprocess, first call and the instance's end,
+// medians: 238 to 292, 18 to 21 and 60 to 63 ms all from the pool, 194 to 220, 16
+// and 33 to 42 so; 218 to 228, 24 and 42 to 47 without a pool; with 16 or 256 MB
+// as the line 199 to 216 and 38 to 42).
 //
 // A buffer may be used on any of the streams that the engine's work runs on
 // (users).  It goes back to the pool, on the pool's own stream, after
@@ -70,6 +76,7 @@ extern thread_local cudaMemPool_t g_dbuf_pool;
 // buffer is held until it can.
 struct DevPool {
   static constexpr uint64_t kKeep = 512ull << 20;
+  static constexpr size_t kDirect = 64ull << 20;
   cudaMemPool_t pool = nullptr;
   cudaStream_t st = nullptr;
   cudaEvent_t ev = nullptr;
@@ -106,9 +113,10 @@ struct DevPool {
   }
   DevPool(const DevPool&) = delete;
   DevPool& operator=(const DevPool&) = delete;
-  // false: the caller asks the device directly (which then has what the pool
-  // did not use)
+  // false: the caller asks the device directly (which, when the pool had no
+  // room, then has what it did not use)
   bool alloc(void** p, size_t bytes) {
+    if (bytes >= kDirect) return false;
     if (!made) make();
     int d = -1;
     if (!pool || cudaGetDevice(&d) != cudaSuccess || d != device) return false;
