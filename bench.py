@@ -49,9 +49,9 @@ WORKLOAD = ("cfg1: 257^3 background (z<0 hexes split into 2 prisms) + 3 spherica
             "65x65x129 (first 4 radial layers split into tets/prisms/pyramids), seed 1")
 REF_LIB = os.path.join(ROOT, "oracle", "_ref", "libtioga_ref.so")
 PORT_LIB = os.path.join(ROOT, "oracle", "_ref", "liboracle.so")
-# DRAM bytes (read + write) of one k_cell_boxes launch per cell, from an ncu
-# capture on the full workload (profiles/k_cell_boxes_cfg1.md).
-CELL_BOX_DRAM_BYTES_PER_CELL = 2235169536 / 26961129  # 82.90 B
+# DRAM bytes (read + write) of one k_cell_boxes launch per cell that it boxes,
+# from an ncu capture on the full workload (profiles/k_cell_boxes_cfg1.md).
+CELL_BOX_DRAM_BYTES_PER_CELL = 832150784 / 9942505  # 83.70 B
 
 
 def cell_box_bytes(system, st):

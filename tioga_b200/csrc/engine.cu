@@ -30,9 +30,10 @@ Engine::Engine() {
   cudaGetDevice(&device_);
   // The side stream's kernels are wide (the hole-map fill fills the device with
   // CTAs) and nothing waits for them before the donor phase, so the main
-  // stream goes first wherever a CTA slot frees up (a batch of 16 systems 1919
-  // us without, 1817 with it).  One step of priority is enough for that, and
-  // leaves the higher ones to the solver's own streams.
+  // stream goes first wherever a CTA slot frees up (a batch of 16 systems,
+  // medians of six processes: 1828 us without, 1733 with it).  One step of
+  // priority is enough for that, and leaves the higher ones to the solver's own
+  // streams.
   int prio_low = 0, prio_high = 0;
   cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
   cudaStreamCreateWithPriority(&own_stream_, cudaStreamNonBlocking, std::max(prio_high, prio_low - 1));
