@@ -591,6 +591,9 @@ int Engine::upload_chunked() {
     TB_CUDA(cudaEventRecord(up_ev_[k], up_));
   }
   const int mb = tune_.cell_box_per_sm;
+  boxes_form_ = -1;  // every leaf is written, whatever becomes of the call
+  groups_culled_ = false;
+  groups_stale_ = true;
   for (int k = 0; k < nch; k++) {
     const long long g0 = (long long)k * up_chunk_, g1 = std::min<long long>(ntot_, g0 + up_chunk_);
     TB_CUDA(cudaStreamWaitEvent(stream_, up_ev_[k], 0));
@@ -625,8 +628,6 @@ int Engine::upload_chunked() {
   gate_valid_ = false;  // the caller may have moved the nodes any way
   boxes_ready_ = true;
   boxes_form_ = 1;
-  groups_culled_ = false;
-  groups_stale_ = true;
   tiles_ready_ = h_up_tile_off_.size() == h_up_leaf_off_.size();
   return 0;
 }

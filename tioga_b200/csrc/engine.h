@@ -585,7 +585,7 @@ class Engine {
   DBuf<int> grp_parts_, grp_act_, blk_bnd_;
   DBuf<unsigned char> grp_live_, part_need_;
   DBuf<float2> part_box_;
-  int boxes_form_ = 1;           // the form the tree's boxes were made for (0: FP64)
+  int boxes_form_ = -1;          // the form the tree's boxes were made for (0: FP64, -1: none whole)
   bool groups_culled_ = false;   // the tree holds the live groups' boxes only
   bool groups_stale_ = false;    // all leaves were boxed since: every group counts as live before the next cull
   DBuf<float4> tnode_;     // 2 per tree node
