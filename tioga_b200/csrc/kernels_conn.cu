@@ -950,7 +950,9 @@ __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restri
     const bool valid = leaf_ok && lane % LC < L.y;
     const long long c = (long long)L.x + lane % LC;
     float f[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    float r[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};  // FORM 0: the tree's
+    double org[3] = {0.0, 0.0, 0.0};  // FORM 0: f is relative to it
+    if (FORM == 0 && leaf_ok)
+      for (int k = 0; k < 3; k++) org[k] = tree_origin(bi[L.w], k);
     if (valid) {
       const int nv = cell_nv[c];
       const int4 c0 = *reinterpret_cast<const int4*>(conn8 + 8 * c);
@@ -972,11 +974,8 @@ __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restri
         o[1] = make_double2(lo[2], hi[0]);
         o[2] = make_double2(hi[1], hi[2]);
         for (int k = 0; k < 3; k++) {
-          f[k] = f_rd(lo[k]);
-          f[k + 3] = f_ru(hi[k]);
-          const double o = tree_origin(bi[L.w], k);
-          r[k] = f_rd(lo[k] - o);
-          r[k + 3] = f_ru(hi[k] - o);
+          f[k] = f_rd(lo[k] - org[k]);
+          f[k + 3] = f_ru(hi[k] - org[k]);
         }
       } else {
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -999,16 +998,17 @@ __global__ void __launch_bounds__(256, MINB) k_cell_boxes(const double* __restri
       for (int k = 0; k < 3; k++) {
         f[k] = fminf(f[k], __shfl_xor_sync(0xffffffffu, f[k], o));
         f[k + 3] = fmaxf(f[k + 3], __shfl_xor_sync(0xffffffffu, f[k + 3], o));
-        if (FORM == 0) {
-          r[k] = fminf(r[k], __shfl_xor_sync(0xffffffffu, r[k], o));
-          r[k + 3] = fmaxf(r[k + 3], __shfl_xor_sync(0xffffffffu, r[k + 3], o));
-        }
       }
     if (leaf_ok && lane % LC == 0) {
       const long long sl = L.z;
-      const float* t = FORM == 0 ? r : f;
-      tnode[2 * sl] = make_float4(t[0], t[1], t[2], t[3]);
-      *reinterpret_cast<float2*>(&tnode[2 * sl + 1]) = make_float2(t[4], t[5]);  // keep the link
+      tnode[2 * sl] = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float2*>(&tnode[2 * sl + 1]) = make_float2(f[4], f[5]);  // keep the link
+      if (FORM == 0)  // the leaf's own box, out of the block's frame; wider by more than the FP64 rounding both ways
+        for (int k = 0; k < 3; k++) {
+          const double a = f[k] + org[k], b = f[k + 3] + org[k];
+          f[k] = f_rd(a - 4.5e-16 * (fabs((double)f[k]) + fabs(a) + fabs(org[k])));
+          f[k + 3] = f_ru(b + 4.5e-16 * (fabs((double)f[k + 3]) + fabs(b) + fabs(org[k])));
+        }
       lbox[2 * leaf] = make_float4(f[0], f[1], f[2], f[3]);
       lbox[2 * leaf + 1] = make_float4(f[4], f[5], __int_as_float(L.w), 0.f);
     }
